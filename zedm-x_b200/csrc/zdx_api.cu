@@ -315,6 +315,10 @@ int stage_in(zdx_ctx* ctx, bool host, const T* src, size_t count, DevBuf& buf, c
 
 }  // namespace
 
+// The call's device counters: totals, queues and flags, then the team rebuild's TEAM_COUNTS ints.
+constexpr int kTeamCounter = 10;
+constexpr int kCounters = kTeamCounter + TEAM_COUNTS / 2;
+
 extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const zdx_mesh_set* ms,
                                  const zdx_pair_batch* pb, zdx_pair_result* out) {
     if (!ctx || !opts || !ms || !pb || !out) return ZDX_ERR_INVALID;
@@ -403,7 +407,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     CK(ctx->buckets.ensure(sizeof(int) * 128));
     CK(ctx->pair_i64.ensure(sizeof(int64_t) * 5 * P1));
     CK(ctx->pair_i32.ensure(sizeof(int32_t) * 6 * P1));
-    CK(ctx->counters.ensure(sizeof(unsigned long long) * 16));
+    CK(ctx->counters.ensure(sizeof(unsigned long long) * kCounters));
     int64_t* pi64 = as<int64_t>(ctx->pair_i64);
     int32_t* pi32 = as<int32_t>(ctx->pair_i32);
     a.pair_seg_off = pi64;
@@ -426,7 +430,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     a.max_nseg = reinterpret_cast<int*>(cnt + 6);
     a.err = reinterpret_cast<int*>(cnt + 7);
     a.seg_total = cnt + 9;
-    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 16, st));
+    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * kCounters, st));
     CK(cudaMemsetAsync(a.pair_status, 0, sizeof(int32_t) * P1, st));
     // optional per-component counts, written by the rebuild stage
     const int64_t comp_cap = out->comp_stats ? std::max<int64_t>(out->comp_stats_cap, 0) : 0;
@@ -558,7 +562,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
         ctape_final = as<int64_t>(ctx->t_cfinal);
     }
 
-    unsigned long long hc[10];
+    unsigned long long hc[kCounters];
     if (plain) {
         ctx->launches += 1 + 2 * NP;
         for (int64_t p = 0; p < NP; ++p) {
@@ -602,35 +606,63 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
                 a.seg_tri = as<int32_t>(ctx->t_segtri);
                 a.seg_cand = as<uint8_t>(ctx->t_segcand);
             }
-            CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 16, st));
+            CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * kCounters, st));
             CK(cudaMemsetAsync(a.pair_status, 0, sizeof(int32_t) * P1, st));
             if (a.pair_done) CK(cudaMemsetAsync(a.pair_done, 0, sizeof(int32_t) * NP, st));
         }
-        // stage 2: rebuild, one warp per pair, slots sized for the largest pair
+        // stage 2: rebuild, by teams in shared memory; the pairs no team holds, every pair of the plain
+        // per-stage form and of polyline's split search, one warp per pair, slots sized for the largest pair
         const int nmax = std::max(((int*)&hc[6])[0], 1);
-        a.k2_nmax = nmax;
-        a.k2_slot_bytes = rebuild_slot_bytes(nmax);
         const size_t budget = (size_t)2 << 30;
-        int64_t warps = std::min<int64_t>(std::max<int64_t>(NP, 1), (int64_t)ctx->num_sms * 32);
-        warps = std::min<int64_t>(warps, std::max<int64_t>(1, (int64_t)(budget / a.k2_slot_bytes)));
-        warps = (warps + ctx->tune.rebuild_warps - 1) / ctx->tune.rebuild_warps * ctx->tune.rebuild_warps;
-        a.k2_nslots = warps;
-        CK(ctx->k2_slots.ensure(a.k2_slot_bytes * (size_t)warps));
-        a.k2_slots = as<char>(ctx->k2_slots);
+        auto warp_form = [&](const int32_t* order, const int64_t pairs) -> int {
+            a.k2_nmax = nmax;
+            a.k2_slot_bytes = rebuild_slot_bytes(nmax);
+            int64_t warps = std::min<int64_t>(std::max<int64_t>(pairs, 1), (int64_t)ctx->num_sms * 32);
+            warps = std::min<int64_t>(warps, std::max<int64_t>(1, (int64_t)(budget / a.k2_slot_bytes)));
+            warps = (warps + ctx->tune.rebuild_warps - 1) / ctx->tune.rebuild_warps * ctx->tune.rebuild_warps;
+            a.k2_nslots = warps;
+            CK(ctx->k2_slots.ensure(a.k2_slot_bytes * (size_t)warps));
+            a.k2_slots = as<char>(ctx->k2_slots);
+            PairArgs w = a;
+            w.order = order;
+            w.item_end = pairs;
+            launch_rebuild(w, (int)warps, ctx->tune.rebuild_warps, st);
+            ctx->launches += 1;
+            return ZDX_OK;
+        };
         const bool arena = ctx->tune.rebuild_arena != 0 && a.mode == 0 && !a.tape_stage && !a.want_pts &&
                            !a.comp_stats && !a.per_stage;
+        const bool teams = !arena && !a.per_stage && (a.mode == 0 || !a.split);
+        TeamPlan plan{};
+        if (teams) {
+            CK(ctx->tm_lists.ensure(sizeof(int32_t) * (TEAM_CLASSES + 1) * P1));
+            plan.lists = as<int32_t>(ctx->tm_lists);
+            plan.stride = (int64_t)P1;
+            plan.counts = reinterpret_cast<int*>(cnt + kTeamCounter);
+        }
         CK(cudaEventRecord(ctx->ev[2], st));
         if (arena) {
             int st_code = rebuild_by_arenas(ctx, a, NP, nmax, budget, st);
             if (st_code != ZDX_OK) return st_code;
+        } else if (teams) {
+            ctx->launches += launch_rebuild_teams(a, plan, ctx->num_sms, NP, nmax, st);
         } else {
-            launch_rebuild(a, (int)warps, ctx->tune.rebuild_warps, st);
-            ctx->launches += 1;
+            int st_code = warp_form(a.order, NP);
+            if (st_code != ZDX_OK) return st_code;
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(ctx->ev[3], st));
         CK(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        const int left = teams ? reinterpret_cast<int*>(hc + kTeamCounter)[TEAM_CLASSES] : 0;
+        if (left > 0) {
+            int st_code = warp_form(plan.lists + TEAM_CLASSES * plan.stride, left);
+            if (st_code != ZDX_OK) return st_code;
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(ctx->ev[3], st));
+            CK(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+        }
     }
     const int err = ((int*)&hc[7])[0];
     ctx->tape_need = (int64_t)hc[8];

@@ -55,6 +55,7 @@ struct zdx_ctx {
     zdx::DevBuf tri_sph, mesh_R, mesh_valid, mesh_infl;
     zdx::DevBuf order, buckets, pair_i64, pair_i32, counters;
     zdx::DevBuf k1_slots, seg_arena, k2_slots;
+    zdx::DevBuf tm_lists;                        // team form of the rebuild: class lists
     zdx::DevBuf ar_lists, ar_counts, ar_gslots;  // arena form of the rebuild: class lists, counts, slots
     zdx::DevBuf sp_items, sp_first, sp_chunk;  // split of large pairs (items, per-pair first item, runs)
     zdx::DevBuf w_scratch;                     // per-item tapes of the wall contacts (zdx_rollout.cu)
@@ -71,7 +72,7 @@ struct zdx_ctx {
 
     std::vector<zdx::DevBuf*> all_bufs() {
         return {&in_tris, &in_off, &in_me, &in_bd, &in_pm, &in_pose, &tri_sph, &mesh_R, &mesh_valid, &mesh_infl,
-                &order, &buckets, &pair_i64, &pair_i32, &counters, &k1_slots, &seg_arena, &k2_slots, &ar_lists,
+                &order, &buckets, &pair_i64, &pair_i32, &counters, &k1_slots, &seg_arena, &k2_slots, &tm_lists, &ar_lists,
                 &ar_counts, &ar_gslots, &sp_items,
                 &sp_first, &sp_chunk, &w_scratch, &p_err,
                 &cstage, &cistage, &pstage, &g_off, &o_cg, &o_ci, &o_pts, &o_cpo, &o_ps, &o_comp, &t_segtri, &t_segcand,

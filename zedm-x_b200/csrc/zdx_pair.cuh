@@ -165,6 +165,18 @@ struct ArenaPlan {
 };
 void launch_rebuild_classes(const PairArgs& a, const ArenaPlan& plan, cudaStream_t s);
 void launch_rebuild_arena(const PairArgs& a, const ArenaPlan& plan, cudaStream_t s);
+// The team form of the rebuild (zdx_team.cuh, zdx_team.cu): the pairs of the order sorted into classes by
+// segment count, one launch a class, everything in shared memory.  Pairs that no class holds are appended to
+// lists[TEAM_CLASSES], for the warp-per-pair kernel.  `most` bounds the pairs, nmax their segments (classes
+// above it are not launched).  Returns the number of kernels launched.
+constexpr int TEAM_CLASSES = 3;
+struct TeamPlan {
+    int32_t* lists;  // TEAM_CLASSES + 1 lists of stride pairs
+    int64_t stride;
+    int* counts;     // TEAM_COUNTS ints, zero before the launch: list lengths, from 8 on the classes' queues
+};
+constexpr int TEAM_COUNTS = 16;
+int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s);
 // Bytes of one triangle-stage slot.
 size_t tritest_slot_bytes(int cap_side, int cap_seg);
 

@@ -1554,7 +1554,8 @@ static int graph_alloc(zdx_ctx* ctx, Scene& s) {
     CKS(G.buckets.ensure(sizeof(int) * 128));
     CKS(G.pair_i64.ensure(sizeof(int64_t) * 5 * P1));
     CKS(G.pair_i32.ensure(sizeof(int32_t) * 6 * P1));
-    CKS(G.counters.ensure(sizeof(unsigned long long) * 16));
+    CKS(G.counters.ensure(sizeof(unsigned long long) * 16 + sizeof(int) * TEAM_COUNTS));
+    CKS(G.tm_lists.ensure(sizeof(int32_t) * (TEAM_CLASSES + 1) * P1));
     G.k1_grid = (int)std::min<int64_t>(P1, (int64_t)ctx->num_sms * ctx->tune.tri_ctas_per_sm);
     CKS(G.k1_slots.ensure(tritest_slot_bytes(max_ntri, G.cap_seg) * (size_t)G.k1_grid));
     CKS(G.seg_arena.ensure(sizeof(double) * 6 * (size_t)std::max<int64_t>(G.segcap, 1)));
@@ -1683,7 +1684,7 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         a.queue2 = reinterpret_cast<int*>(cnt + 5);
         a.max_nseg = reinterpret_cast<int*>(cnt + 6);
         a.err = reinterpret_cast<int*>(cnt + 7);
-        CKS(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 16, st));
+        CKS(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 16 + sizeof(int) * TEAM_COUNTS, st));
         CKS(cudaMemsetAsync(a.pair_status, 0, sizeof(int32_t) * P1, st));
         a.mesh_infl_bits = as<unsigned long long>(G.mesh_infl);  // graph_alloc prepared the meshes
         if (cache) {
@@ -1725,7 +1726,13 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         a.contact_cap = G.ccap;
         a.pts_stage = nullptr;
         a.pts_cap = 0;
-        launch_rebuild(a, G.k2_warps, ctx->tune.rebuild_warps, st);
+        // by teams in shared memory, then the pairs no team holds by a warp each
+        TeamPlan plan{as<int32_t>(G.tm_lists), (int64_t)P1, reinterpret_cast<int*>(cnt + 16)};
+        launch_rebuild_teams(a, plan, ctx->num_sms, G.pcap, G.cap_seg, st);
+        PairArgs rest = a;
+        rest.order = plan.lists + TEAM_CLASSES * plan.stride;
+        rest.order_count = plan.counts + TEAM_CLASSES;
+        launch_rebuild(rest, G.k2_warps, ctx->tune.rebuild_warps, st);
         launch_gather_dev(a, as<int64_t>(G.pr_coff), as<double>(G.pr_geom), as<int32_t>(G.pr_info),
                           as<int32_t>(G.pr_stats), G.scan_tmp.p, st);
         k_g_pair_done<<<1, 1, 0, st>>>(cnt, g);

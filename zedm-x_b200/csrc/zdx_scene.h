@@ -123,7 +123,7 @@ struct GraphStep {
     // clearance cache: sorted pair keys and entries (PairArgs::cache_*), the next step's, per-pair lookups
     DevBuf ckey, cval, ckey2, cval2, cidx, cout, cflag, cscan, chit, chit2, chout, cskip;
     // pair kernels' workspaces
-    DevBuf tri_sph, mesh_R, mesh_valid, mesh_infl, order, buckets, pair_i64, pair_i32, counters, k1_slots, seg_arena, k2_slots,
+    DevBuf tri_sph, mesh_R, mesh_valid, mesh_infl, order, buckets, pair_i64, pair_i32, counters, k1_slots, seg_arena, k2_slots, tm_lists,
         cstage, cistage;
 
     std::vector<DevBuf*> bufs() {
@@ -133,7 +133,7 @@ struct GraphStep {
                 &w_active, &w_scan, &w_pairs, &w_contrib, &w_valid, &w_act, &w_ds, &w_hscan, &w_scratch, &hkey, &hds,
                 &hkey2, &hds2, &whkey, &whds, &whkey2, &whds2, &ckey, &cval, &ckey2, &cval2, &cidx, &cout, &cflag, &chit, &chit2, &chout, &cskip,
                 &cscan, &tri_sph, &mesh_R, &mesh_valid, &mesh_infl, &order, &buckets,
-                &pair_i64, &pair_i32, &counters, &k1_slots, &seg_arena, &k2_slots, &cstage, &cistage};
+                &pair_i64, &pair_i32, &counters, &k1_slots, &seg_arena, &k2_slots, &tm_lists, &cstage, &cistage};
     }
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
