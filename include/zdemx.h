@@ -169,7 +169,7 @@ typedef struct zdx_tuning {
     int32_t tri_ctas_per_sm;    /* triangle-stage CTAs per SM: 1 or 2 (default 2)                     */
     int32_t rebuild_warps;      /* warps per rebuild block, 1..4 (default 4)                          */
     int64_t flat_max;           /* survivor pairs nA' x nB' up to which the flat box test runs rather
-                                   than the hierarchical one (default 8192)                          */
+                                   than the hierarchical one (default 262144)                        */
     int64_t split_tests;        /* a batch with fewer pairs than triangle-stage CTAs splits each pair
                                    of nA x nB triangle tests into ceil(nA nB / split_tests) work items
                                    (at most 64, at most nA) over ranges of A's triangles; 0: never

@@ -384,7 +384,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     a.flat_max = ctx->tune.flat_max;
 
     // stage 0: per-triangle spheres and mesh bounds
-    CK(ctx->tri_sph.ensure(sizeof(double4) * std::max<int64_t>(total_tris, 1)));
+    CK(ctx->tri_sph.ensure((sizeof(double4) + sizeof(float)) * std::max<int64_t>(total_tris, 1)));
     CK(ctx->mesh_R.ensure(sizeof(unsigned long long) * std::max(NM, 1)));
     CK(ctx->mesh_valid.ensure(sizeof(int) * std::max(NM, 1)));
     CK(cudaMemsetAsync(ctx->mesh_R.p, 0, sizeof(unsigned long long) * std::max(NM, 1), st));
@@ -396,6 +396,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     a.mesh_infl_bits = per_stage ? nullptr : as<unsigned long long>(ctx->mesh_infl);
     a.per_stage = per_stage ? 1 : 0;
     a.tri_sph = as<double4>(ctx->tri_sph);
+    a.tri_infl = per_stage ? nullptr : reinterpret_cast<float*>(a.tri_sph + std::max<int64_t>(total_tris, 1));
     a.mesh_R_bits = as<unsigned long long>(ctx->mesh_R);
     a.mesh_valid = as<int>(ctx->mesh_valid);
     launch_mesh_prep(a, total_tris, st);

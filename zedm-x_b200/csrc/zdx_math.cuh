@@ -185,6 +185,52 @@ ZDX_HD bool tri_tri_src(const V3* A, V3 nA, double dA, const V3* B, V3 nB, doubl
     if (src1) *src1 = us[i1];
     return true;
 }
+
+// tri_tri_src in two parts, for callers that spread the six candidates over lanes.  The candidate of edge
+// (p0, p1): its cut with the plane (n, d) of triangle T, if that lies in T.
+ZDX_HD bool tri_cut(V3 p0, V3 p1, V3 T0, V3 T1, V3 T2, V3 n, double d, V3& out) {
+    return seg_plane(p0, p1, n, d, out) && point_in_tri(out, T0, T1, T2, n);
+}
+// The segment of the candidates in `valid` (bit side * 3 + i), pt(c) giving candidate c's point.
+template <class Pt>
+ZDX_HD bool tri_join(V3 nA, V3 nB, unsigned valid, const Pt& pt, V3& o0, V3& o1, int& c0, int& c1) {
+    V3 tau = cross(nA, nB);
+    double lt = norm(tau);
+    if (lt < 1e-20) return false;
+    tau = tau / lt;
+    const double tol2 = 1e-9 * 1e-9;
+    unsigned kept = 0;
+    double min_t = __builtin_huge_val(), max_t = -__builtin_huge_val();
+    int i0 = -1, i1 = -1, nu = 0;
+    for (int c = 0; c < 6; ++c) {
+        if (!(valid >> c & 1u)) continue;
+        const V3 p = pt(c);
+        bool keep = true;
+        for (int k = 0; k < c; ++k)
+            if ((kept >> k & 1u) && norm2(p - pt(k)) <= tol2) keep = false;
+        if (!keep) continue;
+        kept |= 1u << c;
+        ++nu;
+        const double t = dot(p, tau);
+        if (t < min_t) {
+            min_t = t;
+            i0 = c;
+        }
+        if (t > max_t) {
+            max_t = t;
+            i1 = c;
+        }
+    }
+    if (nu < 2 || i0 == i1 || i0 < 0 || i1 < 0) return false;
+    V3 p0 = pt(i0), p1 = pt(i1);
+    if (norm2(p1 - p0) < 1e-18) return false;
+    const bool swap = dot(p1 - p0, tau) < 0.0;
+    o0 = swap ? p1 : p0;
+    o1 = swap ? p0 : p1;
+    c0 = swap ? i1 : i0;
+    c1 = swap ? i0 : i1;
+    return true;
+}
 ZDX_HD bool tri_tri(const V3* A, V3 nA, double dA, const V3* B, V3 nB, double dB, V3& o0, V3& o1) {
     return tri_tri_src(A, nA, dA, B, nB, dB, o0, o1, nullptr, nullptr);
 }

@@ -184,6 +184,63 @@ ZDX_HD_NP bool tri_tri(const double* tA, const double* nA, double dA, const doub
     return true;
 }
 
+// tri_tri in two parts, for callers that spread the six candidates over lanes (tri_cut, tri_join of
+// zdx_math.cuh).  pt(c) gives a pointer to candidate c's point.
+ZDX_HD_NP bool tri_cut(const double* p0, const double* p1, const double* t, const double* n, double d, double* out) {
+    return seg_plane(p0, p1, n, d, out) && point_in_tri(out, t, n);
+}
+template <class Pt>
+ZDX_HD_NP bool tri_join(const double* nA, const double* nB, unsigned valid, const Pt& pt, double* p0, double* p1) {
+    double tau[3];
+    cross3(nA, nB, tau);
+    const double lt = norm3(tau);
+    if (lt < 1e-20) return false;
+    for (int k = 0; k < 3; ++k) tau[k] = tau[k] / lt;
+    unsigned kept = 0;
+    double tmin = 0.0, tmax = 0.0;
+    int i0 = 0, i1 = 0, nc = 0;
+    for (int c = 0; c < 6; ++c) {
+        if (!(valid >> c & 1u)) continue;
+        double p[3], o[3];
+        pt(c, p);
+        bool keep = true;
+        for (int k = 0; k < c; ++k) {
+            if (!(kept >> k & 1u)) continue;
+            pt(k, o);
+            const double df[3] = {p[0] - o[0], p[1] - o[1], p[2] - o[2]};
+            if (norm3(df) <= 1e-9) keep = false;
+        }
+        if (!keep) continue;
+        kept |= 1u << c;
+        const double tc = dot3(p, tau);
+        if (nc == 0) {
+            tmin = tmax = tc;
+            i0 = i1 = c;
+        }
+        if (tc < tmin) {
+            tmin = tc;
+            i0 = c;
+        }
+        if (tc > tmax) {
+            tmax = tc;
+            i1 = c;
+        }
+        ++nc;
+    }
+    if (nc < 2 || i0 == i1) return false;
+    double a[3], b[3];
+    pt(i0, a);
+    pt(i1, b);
+    const double df[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
+    if (norm3(df) < 1e-18) return false;
+    const bool swap = dot3(df, tau) < 0.0;
+    for (int k = 0; k < 3; ++k) {
+        p0[k] = swap ? b[k] : a[k];
+        p1[k] = swap ? a[k] : b[k];
+    }
+    return true;
+}
+
 // ---- polyline.py's rebuild arithmetic
 
 // np.clip(x, 0.0, 1.0): max first, then min, each taking its second operand unless the first is

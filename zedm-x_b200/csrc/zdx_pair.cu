@@ -4,11 +4,13 @@
 // Stage 1  k_segments    persistent CTAs fed by a cost-ordered queue (most expensive pair first).  Per
 //                        pair: cull both triangle lists against the other body's bounding cube (one
 //                        rotation per triangle, conservative so no AABB-overlapping pair is lost),
-//                        transform the survivors exactly as src/main.cpp:499-510 does, test every
-//                        surviving (ta,tb) with the reference's strict AABB compare, queue the overlaps
-//                        in shared memory and run tri_tri_intersection_segment on them with the whole
-//                        CTA, then order the segments by (ta,tb): the reference's emission order.
-// Stage 2  k_rebuild     one warp per pair: components (label_segments_by_contact_greedy), endpoint
+//                        transform the survivors exactly as src/main.cpp:499-510 does, test the boxes of
+//                        every surviving (ta,tb) outward-rounded, list the overlaps, keep those that pass
+//                        the reference's strict AABB compare and that neither triangle's plane rules out,
+//                        run tri_tri_intersection_segment on them (its six candidates over lanes), then
+//                        order the segments by (ta,tb): the reference's emission order.
+// Stage 2  (zdx_team.cu) the rebuild by teams of threads in shared memory; k_rebuild takes what no team holds
+//                        and the plain forms, one warp per pair: components (label_segments_by_contact_greedy), endpoint
 //                        snap, T-junction split, loop trace, Sn/Gn/xc0, filters and the minimal force
 //                        law.  Neighbour scans run across the 32 lanes; decisions whose order the
 //                        reference fixes (DFS pushes, union-find classes, std::sort of ties, the walk)
@@ -29,12 +31,18 @@ namespace zdx {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int K1_THREADS = 256;
-constexpr int K1_ITER = 8;
-constexpr int K1_QCAP = K1_THREADS * K1_ITER;
-constexpr int K1_HCAP = 2048;  // B survivors handled by the hierarchical test (shared memory)
-constexpr size_t K1_DSMEM = sizeof(float) * 6 * K1_HCAP + sizeof(uint32_t) * K1_HCAP + sizeof(int) * K1_HCAP +
-                            sizeof(float) * 6 * (K1_HCAP / 32) + sizeof(int2) * 64 * (K1_THREADS / 32);
-static_assert(sizeof(int2) * K1_QCAP <= (sizeof(uint32_t) + sizeof(int)) * K1_HCAP, "flat queue must fit the alias");
+constexpr int K1_HCAP = 1024;   // B survivors the hierarchical test takes at a time (shared memory)
+constexpr int K1_ATILE = 1024;  // A survivors whose boxes the flat test keeps in shared memory at a time
+constexpr int K1_JOIN = K1_THREADS;  // triangle pairs whose candidate points are in shared memory at a time
+constexpr size_t K1_HBYTES = (sizeof(float) * 6 + sizeof(uint32_t) + sizeof(int)) * K1_HCAP + sizeof(float) * 6 * (K1_HCAP / 32);
+constexpr size_t K1_JBYTES = (sizeof(double) * 18 + sizeof(unsigned)) * K1_JOIN;
+constexpr size_t K1_DSMEM = K1_HBYTES > K1_JBYTES ? K1_HBYTES : K1_JBYTES;
+static_assert(sizeof(float) * 8 * K1_ATILE <= K1_DSMEM, "the flat test's boxes must fit");
+// Entries of a CTA's two lists of triangle pairs (boxes that overlap; those the plane test leaves).
+__host__ __device__ inline int k1_list_cap(int cap) {
+    const int n = 8 * cap;
+    return n < 1024 ? 1024 : (n > 8192 ? 8192 : n);
+}
 
 __device__ __forceinline__ V3 ld3(const double* p) { return V3{p[0], p[1], p[2]}; }
 __device__ __forceinline__ void st3(double* p, V3 v) {
@@ -67,6 +75,7 @@ __global__ void k_mesh_prep(PairArgs a, int64_t total) {
         a.tri_sph[t] = make_double4(c.x, c.y, c.z, r);
         Rb = (unsigned long long)__double_as_longlong((norm(c) + r) * (1.0 + 1e-12));
         valid = !(norm(cross(p1 - p0, p2 - p0)) < 1e-30) ? 1 : 0;
+        if (a.tri_infl && !valid) a.tri_infl[t] = __int_as_float(0x7f800000);
         if (a.mesh_infl_bits && valid) {
             // point_in_tri accepts c_k = |e_k| x (in-plane distance to edge line k) >= -1e-10: each edge line
             // moves out by 1e-10 / |e_k| and a vertex by at most 2 max_k(1e-10 / |e_k|) / sin(its angle)
@@ -78,6 +87,7 @@ __global__ void k_mesh_prep(PairArgs a, int64_t total) {
             double infl = 2.0 * dmax / smin_ang;
             if (!(infl < 1e300)) infl = 1e300;
             ib = (unsigned long long)__double_as_longlong(infl * (1.0 + 1e-6));
+            if (a.tri_infl) a.tri_infl[t] = __double2float_ru(infl * (1.0 + 1e-6));
         }
     }
     // A mesh's triangles are consecutive, so they are runs of lanes: reduce each run (max, sum, max of
@@ -177,6 +187,7 @@ struct K1Side {
 };
 struct K1Slot {
     K1Side side[2];
+    uint2* list[2];  // k1_list_cap(cap): triangle pairs (A survivor, B survivor)
     double* seg;    // 6 x cap_seg
     uint64_t* key;  // cap_seg
     uint8_t* cand;  // 2 x cap_seg: candidate index of each endpoint (adjoint tape)
@@ -195,7 +206,11 @@ __host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, K1S
         d.pl = (double*)take(sizeof(double) * 4 * (size_t)cap);
         d.box = (double*)take(sizeof(double) * 6 * (size_t)cap);
         d.id = (int*)take(sizeof(int) * (size_t)cap);
-        if (s) s->side[k] = d;
+        uint2* l = (uint2*)take(sizeof(uint2) * (size_t)k1_list_cap(cap));
+        if (s) {
+            s->side[k] = d;
+            s->list[k] = l;
+        }
     }
     double* seg = (double*)take(sizeof(double) * 6 * (size_t)cap_seg);
     uint64_t* key = (uint64_t*)take(sizeof(uint64_t) * (size_t)cap_seg);
@@ -229,37 +244,19 @@ __host__ __device__ inline int next_pow2(int n) {
     return p;
 }
 
-// tri_tri_intersection_segment on one queued (A survivor, B survivor) entry; the segment and its
-// (ta, tb) key go to the CTA's segment list.  NPX: in numpy's arithmetic (zdx_npmath.cuh), with no
-// candidate provenance (that mode has no adjoint).
-template <bool NPX>
-__device__ __forceinline__ void eval_entry(const PairArgs& a, const K1Slot& S, const K1Side& SA, const K1Side& SB,
-                                           int cap, int2 e, int* nseg) {
-    V3 TA[3], TB[3];
+// Whether the plane of one triangle (n, d) rules out a segment with another: the other's corners all lie on
+// one side, further than m.  Then no edge of it meets the plane (t is beyond [0, 1] by at least m over the
+// edge, and m covers 1e-10 edges), and no point of the plane lies in it, not even by point_in_tri's
+// tolerance, which moves its edges out by less than m.
+__device__ __forceinline__ bool beyond_plane(const K1Side& P, int p, const K1Side& T, int t, int cap, double m) {
+    const double nx = P.pl[p], ny = P.pl[cap + p], nz = P.pl[2 * cap + p], d = P.pl[3 * cap + p];
+    bool above = true, below = true;
     for (int k = 0; k < 3; ++k) {
-        TA[k] = V3{SA.tri[(3 * k) * cap + e.x], SA.tri[(3 * k + 1) * cap + e.x], SA.tri[(3 * k + 2) * cap + e.x]};
-        TB[k] = V3{SB.tri[(3 * k) * cap + e.y], SB.tri[(3 * k + 1) * cap + e.y], SB.tri[(3 * k + 2) * cap + e.y]};
+        const double s = nx * T.tri[(3 * k) * cap + t] + ny * T.tri[(3 * k + 1) * cap + t] + nz * T.tri[(3 * k + 2) * cap + t] + d;
+        above = above && s > m;
+        below = below && s < -m;
     }
-    V3 na{SA.pl[e.x], SA.pl[cap + e.x], SA.pl[2 * cap + e.x]};
-    V3 nb{SB.pl[e.y], SB.pl[cap + e.y], SB.pl[2 * cap + e.y]};
-    V3 o0, o1;
-    int c0 = 0, c1 = 0;
-    bool hit;
-    if constexpr (NPX) {
-        hit = np::tri_tri(&TA[0].x, &na.x, SA.pl[3 * cap + e.x], &TB[0].x, &nb.x, SB.pl[3 * cap + e.y], &o0.x, &o1.x);
-    } else {
-        hit = tri_tri_src(TA, na, SA.pl[3 * cap + e.x], TB, nb, SB.pl[3 * cap + e.y], o0, o1, &c0, &c1);
-    }
-    if (hit) {
-        int si = atomicAdd(nseg, 1);
-        if (si < a.cap_seg) {
-            st3(S.seg + 6 * si, o0);
-            st3(S.seg + 6 * si + 3, o1);
-            S.key[si] = ((uint64_t)(uint32_t)SA.id[e.x] << 32) | (uint64_t)(uint32_t)SB.id[e.y];
-            S.cand[2 * si] = (uint8_t)c0;
-            S.cand[2 * si + 1] = (uint8_t)c1;
-        }
-    }
+    return above || below;
 }
 
 // |q - q0| or |q + q0|, whichever is smaller (unit quaternions; a rotation and its negative are one)
@@ -274,6 +271,15 @@ __device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned
 
 // CACHE: the clearance cache of a DEM step (PairArgs::cache_*), a separate instantiation so that the
 // others compile as without it.
+//
+// What bounds it: latency (loads of the soups and the survivors, barriers between a pair's phases).  The
+// overlaps of a pair are listed first and taken together: evaluating each 2,048 box tests' overlaps (about 25)
+// at once, a whole tri_tri a lane, kept two of eight warps busy through six candidates in a row.  The planes
+// leave 250 of 600 overlaps on the pair sweep.  Triangle stage on a B200: 65,536-pair sweep 24.3 -> 13.4 ms,
+// 1,500 pairs of 5,120-triangle meshes 2.66 -> 1.41, 6,000 pairs of hulls 1.41 -> 0.78, 64 mixed pairs 0.42 -> 0.23.
+// The flat test up to flat_max survivor pairs: 13.4 ms with 262,144 on the sweep, 14.7 with 8,192 (the line
+// before, when a test cost twice as much), 13.8 without a line; 1.40 against 1.58 ms on the 5,120-triangle pairs
+// (420,000 survivor pairs) with and without.
 template <bool NPX, bool CACHE>
 __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
     __shared__ double sh_red[2][K1_THREADS / 32];
@@ -281,7 +287,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
     __shared__ int sh_sep;
     __shared__ int sh_item;
     __shared__ int sh_n[2];
-    __shared__ int sh_nq;
+    __shared__ int sh_nq, sh_nt;
     __shared__ int sh_nseg;
     __shared__ unsigned long long sh_base;
     __shared__ int sh_last;
@@ -290,17 +296,16 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
     __shared__ unsigned long long sh_cmin, sh_gmin;
     __shared__ int sh_cbad, sh_nh;
     extern __shared__ __align__(16) unsigned char k1_dsm[];
-    // dynamic shared memory: float boxes | keys | values (the flat path's queue aliases keys+values)
-    //                        | group boxes | per-warp overlap queues
+    // dynamic shared memory, one after the other: the hierarchical test's float boxes | keys | values | group
+    // boxes, the flat test's float boxes, the candidate points | valid bits of the triangle pairs
     float* sm_box = reinterpret_cast<float*>(k1_dsm);
     uint32_t* sm_key = reinterpret_cast<uint32_t*>(sm_box + 6 * K1_HCAP);
     int* sm_val = reinterpret_cast<int*>(sm_key + K1_HCAP);
-    int2* sh_q = reinterpret_cast<int2*>(sm_key);
     float* sm_gbox = reinterpret_cast<float*>(sm_val + K1_HCAP);
-    int2* sm_wq = reinterpret_cast<int2*>(sm_gbox + 6 * (K1_HCAP / 32));
     const int tid = threadIdx.x;
     K1Slot S;
-    carve_k1(a.k1_slots + (size_t)blockIdx.x * a.k1_slot_bytes, a.cap_side, a.cap_seg, &S);
+    char* slot = a.k1_slots + (size_t)blockIdx.x * a.k1_slot_bytes;
+    carve_k1(slot, a.cap_side, a.cap_seg, &S);
     const int cap = a.cap_side;
     const bool py = NPX || a.mode == 1;
     const int64_t iend = a.items ? a.item_begin + a.n_items : item_end_of(a);
@@ -310,7 +315,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             sh_item = a.per_stage ? (int)(a.item_begin + blockIdx.x + round * gridDim.x)
                                   : (int)(a.item_begin + atomicAdd(a.queue1, 1));
             sh_n[0] = sh_n[1] = 0;
-            sh_nq = 0;
+            sh_nq = sh_nt = 0;
             sh_nseg = 0;
             if constexpr (CACHE) {
                 sh_cmin = dbits(__builtin_huge_val());
@@ -397,13 +402,17 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                 const bool sep = DA.box[3 * cap + h] < DB.box[h] || DA.box[h] > DB.box[3 * cap + h] ||
                                  DA.box[4 * cap + h] < DB.box[cap + h] || DA.box[cap + h] > DB.box[4 * cap + h] ||
                                  DA.box[5 * cap + h] < DB.box[2 * cap + h] || DA.box[2 * cap + h] > DB.box[5 * cap + h];
-                if (!sep) eval_entry<NPX>(a, S, DA, DB, cap, make_int2(h, h), &sh_nseg);
+                if (!sep) S.list[1][atomicAdd(&sh_nt, 1)] = make_uint2(h, h);
             }
             double* c = a.cache_out + CACHE_W * (int64_t)p;
             for (int k = tid; k < CACHE_W; k += K1_THREADS) c[k] = k == CACHE_SKIP ? 1.0 : e[k];
             for (int h = tid; h < nh; h += K1_THREADS) a.cache_hout[CACHE_H * (int64_t)p + h] = hin[h];
             __syncthreads();
         }
+        // CACHE: the culls keep every triangle within tau more of the other body, so that each triangle
+        // they drop has a clearance of at least tau (the extra survivors meet nothing: the culls are
+        // conservative either way)
+        const double tau = CACHE ? a.cache_tau * (R[0] + R[1]) : 0.0;
         if (!near_only) {
             // Separation certificate along the line of centres d: every point of A lies below the largest
             // corner projection max_v (v.d) of A's triangles, every point of B above B's smallest one.  A
@@ -486,10 +495,6 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             // certificate's argument neither can take part in a segment.
             double cclear = __builtin_huge_val();  // CACHE: smallest clearance of a culled triangle
             bool cbad = false;
-            // CACHE: the culls keep every triangle within tau more of the other body, so that each triangle
-            // they drop has a clearance of at least tau (the extra survivors meet nothing: the culls are
-            // conservative either way)
-            const double tau = CACHE ? a.cache_tau * (R[0] + R[1]) : 0.0;
             for (int s = 0; s < 2; ++s) {
                 const V3 other = tpos[1 - s];
                 const double lim = R[1 - s] + pad;
@@ -584,164 +589,262 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                 if (cbad) sh_cbad = 1;
             }
             __syncthreads();
-            const int nA = sh_n[0], nB = sh_n[1];
-            const int64_t total = (int64_t)nA * nB;
-            const K1Side& SA = S.side[0];
-            const K1Side& SB = S.side[1];
-            // the survivors' exact boxes (component-major, stride cap) stay in the CTA's slot: the tests' gathers
-            // hit in L1, which staging them in shared memory (measured: slower) would take away
-            const double* bA = SA.box;
-            const double* bB = SB.box;
-            const int sA = cap, sB = cap;
-            if (!a.per_stage && nA > 0 && nB > 0 && nB <= K1_HCAP && total > a.flat_max) {
-                // ---- hierarchical test: B's survivors in Morton order, outward-rounded float AABBs and
-                // 32-triangle group boxes in shared memory; one warp per A triangle rejects whole groups
-                // first.  A float reject is exact (the float box contains the double one); every float
-                // overlap is re-tested with the reference's strict double compare.
-                const int N2 = next_pow2(nB);
+        }
+        const int nA = near_only ? 0 : sh_n[0], nB = near_only ? 0 : sh_n[1];
+        const int64_t total = (int64_t)nA * nB;
+        const K1Side& SA = S.side[0];
+        const K1Side& SB = S.side[1];
+        // the survivors' exact boxes (component-major, stride cap) stay in the CTA's slot: the tests' gathers
+        // hit in L1, which staging them in shared memory (measured: slower) would take away
+        const double* bA = SA.box;
+        const double* bB = SB.box;
+        const int sA = cap, sB = cap;
+        const int lcap = k1_list_cap(cap);
+        const int lane = tid & 31, warp = tid >> 5;
+        // the reference's AABB reject (src/main.cpp:2130-2134), strict compares
+        auto meets = [&](int ia, int ib) {
+            return !((bA[3 * sA + ia] < bB[ib]) | (bA[ia] > bB[3 * sB + ib]) | (bA[4 * sA + ia] < bB[sB + ib]) |
+                     (bA[sA + ia] > bB[4 * sB + ib]) | (bA[5 * sA + ia] < bB[2 * sB + ib]) | (bA[2 * sA + ia] > bB[5 * sB + ib]));
+        };
+        auto found = [&](int ia, int ib) {
+            const int q = atomicAdd(&sh_nq, 1);
+            if (q < lcap) S.list[0][q] = make_uint2(ia, ib);
+        };
+        // Windows of survivor pairs, [r0, r1) of A by [c0, c1) of B: all of them at once, unless the pairs found
+        // outgrow the list; then the window is halved and taken again.
+        int r0 = 0, c0 = 0, rows = nA, cols = nB;
+        for (;;) {
+            const int r1 = min(nA, r0 + rows), c1 = min(nB, c0 + cols);
+            const int64_t tests = (int64_t)(r1 - r0) * (c1 - c0);
+            if (!a.per_stage && tests > a.flat_max) {
+                // ---- hierarchical test, B's survivors a tile at a time: the tile in Morton order, outward-rounded
+                // float AABBs and 32-triangle group boxes in shared memory; one warp per A triangle rejects
+                // whole groups first.  A float reject is exact (the float box contains the double one); every
+                // float overlap is tested again below.
                 const double Rb = R[1] + pad;
                 const V3 lo = tpos[1] - V3{Rb, Rb, Rb};
                 const double sc = 1024.0 / (2.0 * Rb);
-                for (int i = tid; i < N2; i += K1_THREADS) {
-                    if (i < nB) {
-                        V3 c{(SB.tri[i] + SB.tri[3 * cap + i] + SB.tri[6 * cap + i]),
-                             (SB.tri[cap + i] + SB.tri[4 * cap + i] + SB.tri[7 * cap + i]),
-                             (SB.tri[2 * cap + i] + SB.tri[5 * cap + i] + SB.tri[8 * cap + i])};
-                        c = c * (1.0 / 3.0);
-                        sm_key[i] = morton3((c.x - lo.x) * sc, (c.y - lo.y) * sc, (c.z - lo.z) * sc);
-                        sm_val[i] = i;
-                    } else {
-                        sm_key[i] = 0xffffffffu;
-                        sm_val[i] = -1;
+                for (int b0 = c0; b0 < c1; b0 += K1_HCAP) {
+                    const int nb = c1 - b0 < K1_HCAP ? c1 - b0 : K1_HCAP;
+                    const int N2 = next_pow2(nb);
+                    if (b0 > c0) __syncthreads();
+                    for (int i = tid; i < N2; i += K1_THREADS) {
+                        if (i < nb) {
+                            const double* T = SB.tri + b0 + i;
+                            V3 c{T[0] + T[3 * cap] + T[6 * cap], T[cap] + T[4 * cap] + T[7 * cap],
+                                 T[2 * cap] + T[5 * cap] + T[8 * cap]};
+                            c = c * (1.0 / 3.0);
+                            sm_key[i] = morton3((c.x - lo.x) * sc, (c.y - lo.y) * sc, (c.z - lo.z) * sc);
+                            sm_val[i] = b0 + i;
+                        } else {
+                            sm_key[i] = 0xffffffffu;
+                            sm_val[i] = -1;
+                        }
                     }
-                }
-                __syncthreads();
-                for (int kk2 = 2; kk2 <= N2; kk2 <<= 1)
-                    for (int j = kk2 >> 1; j > 0; j >>= 1) {
-                        for (int i = tid; i < N2; i += K1_THREADS) {
-                            int ixj = i ^ j;
-                            if (ixj > i) {
-                                bool up = (i & kk2) == 0;
-                                uint32_t ki = sm_key[i], kj = sm_key[ixj];
-                                if ((ki > kj) == up) {
-                                    sm_key[i] = kj;
-                                    sm_key[ixj] = ki;
-                                    int vi = sm_val[i];
-                                    sm_val[i] = sm_val[ixj];
-                                    sm_val[ixj] = vi;
+                    __syncthreads();
+                    for (int kk2 = 2; kk2 <= N2; kk2 <<= 1)
+                        for (int j = kk2 >> 1; j > 0; j >>= 1) {
+                            for (int i = tid; i < N2; i += K1_THREADS) {
+                                int ixj = i ^ j;
+                                if (ixj > i) {
+                                    bool up = (i & kk2) == 0;
+                                    uint32_t ki = sm_key[i], kj = sm_key[ixj];
+                                    if ((ki > kj) == up) {
+                                        sm_key[i] = kj;
+                                        sm_key[ixj] = ki;
+                                        int vi = sm_val[i];
+                                        sm_val[i] = sm_val[ixj];
+                                        sm_val[ixj] = vi;
+                                    }
                                 }
                             }
+                            __syncthreads();
                         }
-                        __syncthreads();
+                    for (int m = tid; m < nb; m += K1_THREADS) {
+                        int ib = sm_val[m];
+                        for (int k = 0; k < 3; ++k) sm_box[k * K1_HCAP + m] = __double2float_rd(bB[k * sB + ib]);
+                        for (int k = 3; k < 6; ++k) sm_box[k * K1_HCAP + m] = __double2float_ru(bB[k * sB + ib]);
                     }
-                for (int m = tid; m < nB; m += K1_THREADS) {
-                    int ib = sm_val[m];
-                    for (int k = 0; k < 3; ++k) sm_box[k * K1_HCAP + m] = __double2float_rd(bB[k * sB + ib]);
-                    for (int k = 3; k < 6; ++k) sm_box[k * K1_HCAP + m] = __double2float_ru(bB[k * sB + ib]);
-                }
-                __syncthreads();
-                const int ng = (nB + 31) >> 5;
-                const int lane = tid & 31, warp = tid >> 5;
-                for (int g = warp; g < ng; g += K1_THREADS / 32) {
-                    int m = g * 32 + lane;
-                    float v[6];
-                    for (int k = 0; k < 3; ++k) v[k] = m < nB ? sm_box[k * K1_HCAP + m] : __int_as_float(0x7f800000);
-                    for (int k = 3; k < 6; ++k) v[k] = m < nB ? sm_box[k * K1_HCAP + m] : -__int_as_float(0x7f800000);
-                    for (int o = 16; o > 0; o >>= 1) {
-                        for (int k = 0; k < 3; ++k) v[k] = fminf(v[k], __shfl_xor_sync(FULL, v[k], o));
-                        for (int k = 3; k < 6; ++k) v[k] = fmaxf(v[k], __shfl_xor_sync(FULL, v[k], o));
-                    }
-                    if (lane < 6) sm_gbox[lane * (K1_HCAP / 32) + g] = v[lane];
-                }
-                __syncthreads();
-                int2* wq = sm_wq + warp * 64;
-                int wq_n = 0;
-                for (int ia = warp; ia < nA; ia += K1_THREADS / 32) {
-                    double da[6];
-                    for (int k = 0; k < 6; ++k) da[k] = bA[k * sA + ia];
-                    float fa[6];
-                    for (int k = 0; k < 3; ++k) fa[k] = __double2float_rd(da[k]);
-                    for (int k = 3; k < 6; ++k) fa[k] = __double2float_ru(da[k]);
-                    for (int gb = 0; gb < ng; gb += 32) {
-                        const int g = gb + lane;
-                        bool ov = false;
-                        if (g < ng) {
-                            const float* G = sm_gbox + g;
-                            const int gs = K1_HCAP / 32;
-                            ov = !(fa[3] < G[0] || fa[0] > G[3 * gs] || fa[4] < G[gs] || fa[1] > G[4 * gs] ||
-                                   fa[5] < G[2 * gs] || fa[2] > G[5 * gs]);
+                    __syncthreads();
+                    const int ng = (nb + 31) >> 5;
+                    for (int g = warp; g < ng; g += K1_THREADS / 32) {
+                        int m = g * 32 + lane;
+                        float v[6];
+                        for (int k = 0; k < 3; ++k) v[k] = m < nb ? sm_box[k * K1_HCAP + m] : __int_as_float(0x7f800000);
+                        for (int k = 3; k < 6; ++k) v[k] = m < nb ? sm_box[k * K1_HCAP + m] : -__int_as_float(0x7f800000);
+                        for (int o = 16; o > 0; o >>= 1) {
+                            for (int k = 0; k < 3; ++k) v[k] = fminf(v[k], __shfl_xor_sync(FULL, v[k], o));
+                            for (int k = 3; k < 6; ++k) v[k] = fmaxf(v[k], __shfl_xor_sync(FULL, v[k], o));
                         }
-                        unsigned gbal = __ballot_sync(FULL, ov);
+                        if (lane < 6) sm_gbox[lane * (K1_HCAP / 32) + g] = v[lane];
+                    }
+                    __syncthreads();
+                    static_assert(K1_HCAP <= 32 * 32, "a tile's groups are one to a lane");
+                    for (int ia = r0 + warp; ia < r1; ia += K1_THREADS / 32) {
+                        float fa[6];
+                        for (int k = 0; k < 3; ++k) fa[k] = __double2float_rd(bA[k * sA + ia]);
+                        for (int k = 3; k < 6; ++k) fa[k] = __double2float_ru(bA[k * sA + ia]);
+                        // all six compares at once: a chain of short-circuits waits out a load for each
+                        auto apart = [&](const float* B, int st) {
+                            return bool((fa[3] < B[0]) | (fa[0] > B[3 * st]) | (fa[4] < B[st]) | (fa[1] > B[4 * st]) |
+                                        (fa[5] < B[2 * st]) | (fa[2] > B[5 * st]));
+                        };
+                        unsigned gbal = __ballot_sync(FULL, lane < ng && !apart(sm_gbox + lane, K1_HCAP / 32));
                         while (gbal) {
-                            const int gg = gb + __ffs(gbal) - 1;
+                            const int m = (__ffs(gbal) - 1) * 32 + lane;
                             gbal &= gbal - 1u;
-                            const int m = gg * 32 + lane;
-                            bool hit = false;
-                            int ib = 0;
-                            if (m < nB) {
-                                const float* Bm = sm_box + m;
-                                bool fov = !(fa[3] < Bm[0] || fa[0] > Bm[3 * K1_HCAP] || fa[4] < Bm[K1_HCAP] ||
-                                             fa[1] > Bm[4 * K1_HCAP] || fa[5] < Bm[2 * K1_HCAP] || fa[2] > Bm[5 * K1_HCAP]);
-                                if (fov) {
-                                    ib = sm_val[m];
-                                    // the reference's AABB reject (src/main.cpp:2130-2134), strict compares
-                                    hit = !(da[3] < bB[ib] || da[0] > bB[3 * sB + ib] || da[4] < bB[sB + ib] ||
-                                            da[1] > bB[4 * sB + ib] || da[5] < bB[2 * sB + ib] || da[2] > bB[5 * sB + ib]);
-                                }
-                            }
-                            unsigned hb = __ballot_sync(FULL, hit);
-                            if (hit) wq[wq_n + __popc(hb & ((1u << lane) - 1u))] = make_int2(ia, ib);
-                            wq_n += __popc(hb);
-                            if (wq_n >= 32) {
-                                __syncwarp();
-                                for (int q = lane; q < wq_n; q += 32) eval_entry<NPX>(a, S, SA, SB, cap, wq[q], &sh_nseg);
-                                __syncwarp();
-                                wq_n = 0;
-                            }
+                            if (m < nb && !apart(sm_box + m, K1_HCAP)) found(ia, sm_val[m]);
                         }
                     }
                 }
-                __syncwarp();
-                for (int q = lane; q < wq_n; q += 32) eval_entry<NPX>(a, S, SA, SB, cap, wq[q], &sh_nseg);
-                __syncthreads();
-            } else if (nB > 0) {
-                int ia = 0, ib = 0, dA = 0, dB = 0;
-                if (nB > 0) {
-                    ia = tid / nB;
-                    ib = tid % nB;
-                    dA = K1_THREADS / nB;
-                    dB = K1_THREADS % nB;
-                }
-                for (int64_t base = 0; base < total; base += K1_QCAP) {
-        #pragma unroll 1
-                    for (int it = 0; it < K1_ITER; ++it) {
-                        int64_t kk = base + (int64_t)it * K1_THREADS + tid;
-                        if (kk < total) {
-                            // the reference's AABB reject (src/main.cpp:2130-2134), strict compares
-                            bool sep = bA[3 * sA + ia] < bB[0 * sB + ib] || bA[0 * sA + ia] > bB[3 * sB + ib] ||
-                                       bA[4 * sA + ia] < bB[1 * sB + ib] || bA[1 * sA + ia] > bB[4 * sB + ib] ||
-                                       bA[5 * sA + ia] < bB[2 * sB + ib] || bA[2 * sA + ia] > bB[5 * sB + ib];
-                            if (!sep) {
-                                int qi = atomicAdd(&sh_nq, 1);
-                                sh_q[qi] = make_int2(ia, ib);
-                            }
-                        }
-                        ib += dB;
-                        ia += dA;
-                        if (ib >= nB) {
-                            ib -= nB;
-                            ia++;
-                        }
+            } else if (!a.per_stage && tests > 0) {
+                // ---- flat test: A's boxes, rounded outward to float, in shared memory (read by every lane at
+                // once), 32 of B's in a warp's lanes; a float overlap is tested again below
+                float4* bx = reinterpret_cast<float4*>(sm_box);
+                for (int a0 = r0; a0 < r1; a0 += K1_ATILE) {
+                    const int na = r1 - a0 < K1_ATILE ? r1 - a0 : K1_ATILE;
+                    if (a0 > r0) __syncthreads();
+                    for (int i = tid; i < na; i += K1_THREADS) {
+                        const double* b = bA + a0 + i;
+                        bx[2 * i] = make_float4(__double2float_rd(b[0]), __double2float_rd(b[sA]),
+                                                __double2float_rd(b[2 * sA]), __double2float_ru(b[3 * sA]));
+                        bx[2 * i + 1] = make_float4(__double2float_ru(b[4 * sA]), __double2float_ru(b[5 * sA]), 0.f, 0.f);
                     }
                     __syncthreads();
-                    const int nq = sh_nq;
-                    for (int qi = tid; qi < nq; qi += K1_THREADS) eval_entry<NPX>(a, S, SA, SB, cap, sh_q[qi], &sh_nseg);
-                    __syncthreads();
-                    if (tid == 0) sh_nq = 0;
-                    __syncthreads();
+                    // a warp's unit: 32 of A against 32 of B
+                    const int ua = (na + 31) >> 5, ub = (c1 - c0 + 31) >> 5;
+                    for (int u = warp; u < ua * ub; u += K1_THREADS / 32) {
+                        const int ib = c0 + (u % ub) * 32 + lane;
+                        const double* b = bB + (ib < c1 ? ib : c1 - 1);
+                        float x0 = __double2float_rd(b[0]), y0 = __double2float_rd(b[sB]), z0 = __double2float_rd(b[2 * sB]);
+                        float x1 = __double2float_ru(b[3 * sB]), y1 = __double2float_ru(b[4 * sB]),
+                              z1 = __double2float_ru(b[5 * sB]);
+                        if (ib >= c1) x0 = __int_as_float(0x7f800000), x1 = -x0;  // no box meets it
+                        const int i0 = (u / ub) * 32, i1 = i0 + 32 < na ? i0 + 32 : na;
+#pragma unroll 4
+                        for (int i = i0; i < i1; ++i) {
+                            const float4 p = bx[2 * i];
+                            const float2 q = *reinterpret_cast<const float2*>(bx + 2 * i + 1);
+                            // all six compares at once: a chain of short-circuits branches after each
+                            const bool apart = (p.w < x0) | (p.x > x1) | (q.x < y0) | (p.y > y1) | (q.y < z0) | (p.z > z1);
+                            if (!apart) found(a0 + i, ib);
+                        }
+                    }
+                }
+            } else {
+                // the plain per-stage form: every pair given the reference's strict FP64 test
+                for (int64_t kk = tid; kk < tests; kk += K1_THREADS) {
+                    const int ia = r0 + (int)(kk / (c1 - c0)), ib = c0 + (int)(kk % (c1 - c0));
+                    if (meets(ia, ib)) found(ia, ib);
                 }
             }
-            if constexpr (CACHE) {
+            __syncthreads();
+            const int nq = sh_nq;
+            if (nq > lcap) {
+                if (rows > 1) rows = (rows + 1) >> 1;
+                else cols = (cols + 1) >> 1;
+                __syncthreads();
+                if (tid == 0) sh_nq = 0;
+                __syncthreads();
+                continue;
+            }
+            // ---- the listed pairs: the reference's box test, then the planes
+            for (int q = tid; q < nq; q += K1_THREADS) {
+                const uint2 e = S.list[0][q];
+                if (!meets(e.x, e.y)) continue;
+                if (a.tri_infl) {
+                    const double more = 8.0 * pad;
+                    const bool far0 = beyond_plane(SB, e.y, SA, e.x, cap, a.tri_infl[off[0] + SA.id[e.x]] + more);
+                    const bool far1 = beyond_plane(SA, e.x, SB, e.y, cap, a.tri_infl[off[1] + SB.id[e.y]] + more);
+                    if (far0 | far1) continue;
+                }
+                S.list[1][atomicAdd(&sh_nt, 1)] = e;
+            }
+            __syncthreads();
+            // ---- tri_tri on the pairs left (src/main.cpp:579-631): its six edge-plane candidates over lanes, then the
+            // segment of a pair's candidates by one lane.  (Whole tri_tri calls, a lane each, kept two of eight
+            // warps waiting on six candidates in a row.)
+            {
+                const int nt2 = sh_nt;
+                double* cut = reinterpret_cast<double*>(k1_dsm);  // candidate c, coordinate k of pair j: (3c + k) K1_JOIN + j
+                unsigned* valid = reinterpret_cast<unsigned*>(cut + 18 * K1_JOIN);
+                for (int q0 = 0; q0 < nt2; q0 += K1_JOIN) {
+                    const int nj = nt2 - q0 < K1_JOIN ? nt2 - q0 : K1_JOIN;
+                    __syncthreads();
+                    for (int j = tid; j < nj; j += K1_THREADS) valid[j] = 0u;
+                    __syncthreads();
+                    for (int x = tid; x < 6 * nj; x += K1_THREADS) {
+                        const int j = x / 6, c = x - 6 * j;
+                        const uint2 e = S.list[1][q0 + j];
+                        const bool sb = c >= 3;  // an edge of B against A's plane
+                        const int i = sb ? c - 3 : c, i2 = i == 2 ? 0 : i + 1;
+                        const double* E = (sb ? S.side[1].tri + e.y : S.side[0].tri + e.x);
+                        const double* T = (sb ? S.side[0].tri + e.x : S.side[1].tri + e.y);
+                        const double* P = (sb ? S.side[0].pl + e.x : S.side[1].pl + e.y);
+                        auto corner = [&](const double* t, int k) { return V3{t[3 * k * cap], t[(3 * k + 1) * cap], t[(3 * k + 2) * cap]}; };
+                        const V3 n{P[0], P[cap], P[2 * cap]};
+                        const V3 p0 = corner(E, i), p1 = corner(E, i2);
+                        V3 o;
+                        bool ok;
+                        if constexpr (NPX) {
+                            const V3 t3[3] = {corner(T, 0), corner(T, 1), corner(T, 2)};
+                            ok = np::tri_cut(&p0.x, &p1.x, &t3[0].x, &n.x, P[3 * cap], &o.x);
+                        } else {
+                            ok = tri_cut(p0, p1, corner(T, 0), corner(T, 1), corner(T, 2), n, P[3 * cap], o);
+                        }
+                        if (ok) {
+                            cut[(3 * c) * K1_JOIN + j] = o.x;
+                            cut[(3 * c + 1) * K1_JOIN + j] = o.y;
+                            cut[(3 * c + 2) * K1_JOIN + j] = o.z;
+                            atomicOr(valid + j, 1u << c);
+                        }
+                    }
+                    __syncthreads();
+                    for (int j = tid; j < nj; j += K1_THREADS) {
+                        const unsigned v = valid[j];
+                        if (__popc(v) < 2) continue;
+                        const uint2 e = S.list[1][q0 + j];
+                        const V3 na{S.side[0].pl[e.x], S.side[0].pl[cap + e.x], S.side[0].pl[2 * cap + e.x]};
+                        const V3 nb{S.side[1].pl[e.y], S.side[1].pl[cap + e.y], S.side[1].pl[2 * cap + e.y]};
+                        V3 o0, o1;
+                        int c0 = 0, c1 = 0;
+                        bool hit;
+                        if constexpr (NPX) {
+                            auto pt = [&](int c, double* p) {
+                                for (int k = 0; k < 3; ++k) p[k] = cut[(3 * c + k) * K1_JOIN + j];
+                            };
+                            hit = np::tri_join(&na.x, &nb.x, v, pt, &o0.x, &o1.x);
+                        } else {
+                            auto pt = [&](int c) {
+                                return V3{cut[(3 * c) * K1_JOIN + j], cut[(3 * c + 1) * K1_JOIN + j], cut[(3 * c + 2) * K1_JOIN + j]};
+                            };
+                            hit = tri_join(na, nb, v, pt, o0, o1, c0, c1);
+                        }
+                        if (hit) {
+                            const int si = atomicAdd(&sh_nseg, 1);
+                            if (si < a.cap_seg) {
+                                st3(S.seg + 6 * si, o0);
+                                st3(S.seg + 6 * si + 3, o1);
+                                S.key[si] = ((uint64_t)(uint32_t)S.side[0].id[e.x] << 32) | (uint64_t)(uint32_t)S.side[1].id[e.y];
+                                S.cand[2 * si] = (uint8_t)c0;
+                                S.cand[2 * si + 1] = (uint8_t)c1;
+                            }
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+            c0 = c1;
+            if (c0 >= nB) {
+                c0 = 0;
+                r0 = r1;
+            }
+            if (r0 >= nA || nB == 0) break;
+            if (tid == 0) sh_nq = sh_nt = 0;
+            __syncthreads();
+        }
+        if constexpr (CACHE) {
+            if (!near_only) {
                 // the pair's clearance: none with a triangle without a plane.  Survivor pairs whose boxes are
                 // less than tau apart (those that met, and so every segment, included) become the entry's near pairs,
                 // tested again at every skip; the clearance is the smallest of the culled triangles' and of
@@ -780,7 +883,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                 if (tid == CACHE_NH) c[CACHE_NH] = (double)(sh_nh < CACHE_H ? sh_nh : CACHE_H);
                 if (tid > CACHE_NH && tid < CACHE_W) c[tid] = 0.0;
             }
-        }
+                }
         int ns = sh_nseg;
         int status = 0;
         if (ns > a.cap_seg) {

@@ -1546,7 +1546,7 @@ static int graph_alloc(zdx_ctx* ctx, Scene& s) {
     CKS(cudaMemsetAsync(&as<GraphCounts>(G.g)->ncache, 0, sizeof(int64_t), ctx->stream));
     // pair kernels
     const int64_t total_tris = s.mesh_off.back();
-    CKS(G.tri_sph.ensure(sizeof(double4) * (size_t)std::max<int64_t>(total_tris, 1)));
+    CKS(G.tri_sph.ensure((sizeof(double4) + sizeof(float)) * (size_t)std::max<int64_t>(total_tris, 1)));
     CKS(G.mesh_R.ensure(sizeof(unsigned long long) * std::max(nm, 1)));
     CKS(G.mesh_valid.ensure(sizeof(int) * std::max(nm, 1)));
     CKS(G.mesh_infl.ensure(sizeof(unsigned long long) * std::max(nm, 1)));
@@ -1575,6 +1575,7 @@ static int graph_alloc(zdx_ctx* ctx, Scene& s) {
         m.tris = as<double>(s.d_mtris);
         m.tri_off = as<int64_t>(s.d_moff);
         m.tri_sph = as<double4>(G.tri_sph);
+        m.tri_infl = reinterpret_cast<float*>(m.tri_sph + std::max<int64_t>(total_tris, 1));
         m.mesh_R_bits = as<unsigned long long>(G.mesh_R);
         m.mesh_valid = as<int>(G.mesh_valid);
         m.mesh_infl_bits = as<unsigned long long>(G.mesh_infl);
@@ -1646,6 +1647,7 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         a.mean_edge = as<double>(s.d_mme);
         a.bbox_diag = as<double>(s.d_mbd);
         a.tri_sph = as<double4>(G.tri_sph);
+        a.tri_infl = reinterpret_cast<float*>(a.tri_sph + std::max<int64_t>(s.mesh_off.back(), 1));
         a.mesh_R_bits = as<unsigned long long>(G.mesh_R);
         a.mesh_valid = as<int>(G.mesh_valid);
         a.n_pairs = G.pcap;

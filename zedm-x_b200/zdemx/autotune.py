@@ -32,7 +32,7 @@ import numpy as np
 from . import _lib
 
 GRID = {
-    "flat_max": (0, 2048, 8192, 32768, 131072),
+    "flat_max": (0, 8192, 65536, 262144, 1048576),
     "tri_ctas_per_sm": (1, 2),
     "rebuild_warps": (1, 2, 4),
     "split_tests": (0, 16384, 131072),
@@ -40,7 +40,7 @@ GRID = {
     "arena_warps": (4, 8, 12, 16),
     "arena_min_seg": (96, 192, 384),
 }
-DEFAULTS = {"tri_ctas_per_sm": 2, "rebuild_warps": 4, "flat_max": 8192, "split_tests": 0, "rebuild_arena": 0,
+DEFAULTS = {"tri_ctas_per_sm": 2, "rebuild_warps": 4, "flat_max": 262144, "split_tests": 0, "rebuild_arena": 0,
             "arena_warps": 8, "arena_min_seg": 192}
 
 
