@@ -382,6 +382,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     a.cap_seg = opts->max_seg_per_pair > 0 ? opts->max_seg_per_pair : 16384;
     a.cap_side = std::max(max_ntri, 1);
     a.flat_max = ctx->tune.flat_max;
+    a.k1_threads = opts->sched == ZDX_SCHED_PLAIN ? 256 : triangle_threads(max_ntri, NP, ctx->num_sms, a.mode);
 
     // stage 0: per-triangle spheres and mesh bounds
     CK(ctx->tri_sph.ensure((sizeof(double4) + sizeof(float)) * std::max<int64_t>(total_tris, 1)));
@@ -463,11 +464,11 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     ctx->launches += plain ? 0 : per_stage ? 1 : 4;  // mesh prep (+ three cost-order kernels)
 
     // stage 1: segments
-    int k1_grid = plain ? 1 : (int)std::min<int64_t>(std::max<int64_t>(NP, 1), (int64_t)ctx->num_sms * ctx->tune.tri_ctas_per_sm);
+    int k1_grid = plain ? 1 : (int)std::min<int64_t>(std::max<int64_t>(NP, 1), (int64_t)ctx->num_sms * triangle_ctas(ctx->tune.tri_ctas_per_sm, a.k1_threads));
     // A batch with fewer pairs than triangle-stage CTAs splits its large pairs: a pair of nA x nB triangle
     // tests becomes ceil(nA nB / split_tests) work items (at most 64, at most nA), each over a range of A's
     // triangles, joined back in order on the device.  The items go most expensive pair first.
-    const int64_t ctas = (int64_t)ctx->num_sms * ctx->tune.tri_ctas_per_sm;
+    const int64_t ctas = (int64_t)ctx->num_sms * triangle_ctas(ctx->tune.tri_ctas_per_sm, a.k1_threads);
     if (!plain && !per_stage && ctx->tune.split_tests > 0 && NP > 0 && NP < ctas) {
         std::vector<int32_t> pm_h((size_t)(2 * NP));
         if (host) {

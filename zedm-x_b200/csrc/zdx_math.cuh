@@ -231,6 +231,28 @@ ZDX_HD bool tri_join(V3 nA, V3 nB, unsigned valid, const Pt& pt, V3& o0, V3& o1,
     c1 = swap ? i0 : i1;
     return true;
 }
+// How far outside triangle (p0, p1, p2) point_in_tri can accept a point: it accepts c_k = |e_k| x (in-plane distance
+// to edge line k) >= -1e-10, so each edge line moves out by 1e-10 / |e_k| and a vertex by at most
+// 2 max_k(1e-10 / |e_k|) / sin(its angle).
+ZDX_HD double tri_inflation(V3 p0, V3 p1, V3 p2) {
+    const V3 e0 = p1 - p0, e1 = p2 - p1, e2 = p0 - p2;
+    const double l0 = norm(e0), l1 = norm(e1), l2 = norm(e2);
+    const double cr = norm(cross(e0, e2));
+    const double smin_ang = smin3(cr / (l0 * l2), cr / (l0 * l1), cr / (l1 * l2));
+    const double dmax = 1e-10 / smin3(l0, l1, l2);
+    double infl = 2.0 * dmax / smin_ang;
+    if (!(infl < 1e300)) infl = 1e300;
+    return infl * (1.0 + 1e-6);
+}
+// Whether the plane (n, d) of one triangle rules out a segment with triangle (a, b, c): its corners all lie on one
+// side, further than m.  Then no edge of it meets the plane (t is beyond [0, 1] by at least m over the edge, and m
+// covers 1e-10 edges), and no point of the plane lies in it, not even by point_in_tri's tolerance, which moves its
+// edges out by less than m.
+ZDX_HD bool beyond_plane(V3 n, double d, V3 a, V3 b, V3 c, double m) {
+    const double s0 = n.x * a.x + n.y * a.y + n.z * a.z + d, s1 = n.x * b.x + n.y * b.y + n.z * b.z + d,
+                 s2 = n.x * c.x + n.y * c.y + n.z * c.z + d;
+    return ((s0 > m) & (s1 > m) & (s2 > m)) | ((s0 < -m) & (s1 < -m) & (s2 < -m));
+}
 ZDX_HD bool tri_tri(const V3* A, V3 nA, double dA, const V3* B, V3 nB, double dB, V3& o0, V3& o1) {
     return tri_tri_src(A, nA, dA, B, nB, dB, o0, o1, nullptr, nullptr);
 }

@@ -30,14 +30,21 @@
 namespace zdx {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int K1_THREADS = 256;
-constexpr int K1_HCAP = 1024;   // B survivors the hierarchical test takes at a time (shared memory)
-constexpr int K1_ATILE = 1024;  // A survivors whose boxes the flat test keeps in shared memory at a time
-constexpr int K1_JOIN = K1_THREADS;  // triangle pairs whose candidate points are in shared memory at a time
-constexpr size_t K1_HBYTES = (sizeof(float) * 6 + sizeof(uint32_t) + sizeof(int)) * K1_HCAP + sizeof(float) * 6 * (K1_HCAP / 32);
-constexpr size_t K1_JBYTES = (sizeof(double) * 18 + sizeof(unsigned)) * K1_JOIN;
-constexpr size_t K1_DSMEM = K1_HBYTES > K1_JBYTES ? K1_HBYTES : K1_JBYTES;
-static_assert(sizeof(float) * 8 * K1_ATILE <= K1_DSMEM, "the flat test's boxes must fit");
+// The triangle stage's block of T threads: what of a pair is in shared memory at a time, and the CTAs an SM holds.
+template <int T>
+struct K1 {
+    static constexpr int HCAP = 4 * T;  // B survivors the hierarchical test takes at a time
+    static constexpr int BCAP = 4 * T;  // survivors of a side whose boxes the flat test keeps
+    static constexpr int JOIN = T;      // triangle pairs whose candidate points are there
+    static constexpr size_t HBYTES = (sizeof(float) * 6 + sizeof(uint32_t) + sizeof(int)) * HCAP + sizeof(float) * 6 * (HCAP / 32);
+    static constexpr size_t JBYTES = (sizeof(double) * 18 + sizeof(unsigned)) * JOIN;
+    static constexpr size_t BBYTES = (sizeof(float4) + sizeof(float2)) * 2 * BCAP;
+    static constexpr size_t BYTES = HBYTES > JBYTES ? (HBYTES > BBYTES ? HBYTES : BBYTES) : (JBYTES > BBYTES ? JBYTES : BBYTES);
+    // The kernel waits on memory and barriers more than it issues (a third of the slots with 16 warps an SM), so
+    // 24 warps pay for the registers they take (80 instead of 128): 13.4 -> 10.4 ms on the pair sweep; 32 warps
+    // (64 registers) 10.8.
+    static constexpr int RESIDENT = 768 / T;
+};
 // Entries of a CTA's two lists of triangle pairs (boxes that overlap; those the plane test leaves).
 __host__ __device__ inline int k1_list_cap(int cap) {
     const int n = 8 * cap;
@@ -77,17 +84,9 @@ __global__ void k_mesh_prep(PairArgs a, int64_t total) {
         valid = !(norm(cross(p1 - p0, p2 - p0)) < 1e-30) ? 1 : 0;
         if (a.tri_infl && !valid) a.tri_infl[t] = __int_as_float(0x7f800000);
         if (a.mesh_infl_bits && valid) {
-            // point_in_tri accepts c_k = |e_k| x (in-plane distance to edge line k) >= -1e-10: each edge line
-            // moves out by 1e-10 / |e_k| and a vertex by at most 2 max_k(1e-10 / |e_k|) / sin(its angle)
-            const V3 e0 = p1 - p0, e1 = p2 - p1, e2 = p0 - p2;
-            const double l0 = norm(e0), l1 = norm(e1), l2 = norm(e2);
-            const double cr = norm(cross(e0, e2));
-            const double smin_ang = smin3(cr / (l0 * l2), cr / (l0 * l1), cr / (l1 * l2));
-            const double dmax = 1e-10 / smin3(l0, l1, l2);
-            double infl = 2.0 * dmax / smin_ang;
-            if (!(infl < 1e300)) infl = 1e300;
-            ib = (unsigned long long)__double_as_longlong(infl * (1.0 + 1e-6));
-            if (a.tri_infl) a.tri_infl[t] = __double2float_ru(infl * (1.0 + 1e-6));
+            const double infl = tri_inflation(p0, p1, p2);
+            ib = (unsigned long long)__double_as_longlong(infl);
+            if (a.tri_infl) a.tri_infl[t] = __double2float_ru(infl);
         }
     }
     // A mesh's triangles are consecutive, so they are runs of lanes: reduce each run (max, sum, max of
@@ -182,7 +181,6 @@ void launch_cost_order(const PairArgs& a, int32_t* order, int* buckets, cudaStre
 struct K1Side {
     double* tri;  // 9 x cap, component-major
     double* pl;   // 4 x cap: nx ny nz d
-    double* box;  // 6 x cap: min xyz, max xyz
     int* id;      // cap
 };
 struct K1Slot {
@@ -204,7 +202,6 @@ __host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, K1S
         K1Side d;
         d.tri = (double*)take(sizeof(double) * 9 * (size_t)cap);
         d.pl = (double*)take(sizeof(double) * 4 * (size_t)cap);
-        d.box = (double*)take(sizeof(double) * 6 * (size_t)cap);
         d.id = (int*)take(sizeof(int) * (size_t)cap);
         uint2* l = (uint2*)take(sizeof(uint2) * (size_t)k1_list_cap(cap));
         if (s) {
@@ -223,6 +220,14 @@ __host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, K1S
     return off;
 }
 
+// Meshes of up to 1,280 triangles leave a block of 256 half idle in most of a pair's phases: blocks of 128, twice as
+// many, take 0.74 against 0.95 ms on 16,384 pairs of 320-triangle meshes, 26.9 against 28.3 ms for ten steps of a
+// 30,000-particle pour (124 to 1,280 triangles), and 1.55 against 1.23 ms on 1,500 pairs of 5,120.  A batch that
+// gives an SM less than six pairs wants the larger block for each (64 mixed pairs: 0.26 against 0.50 ms).
+int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode) {
+    return mode != 2 && max_ntri <= 1280 && pairs >= 6 * (int64_t)sms ? 128 : 256;
+}
+int triangle_ctas(int knob, int threads) { return knob >= 2 ? (threads == 128 ? K1<128>::RESIDENT : K1<256>::RESIDENT) : 1; }
 size_t tritest_slot_bytes(int cap_side, int cap_seg) { return carve_k1(nullptr, cap_side, cap_seg, nullptr); }
 
 __device__ __forceinline__ uint32_t expand10(uint32_t v) {
@@ -244,19 +249,16 @@ __host__ __device__ inline int next_pow2(int n) {
     return p;
 }
 
-// Whether the plane of one triangle (n, d) rules out a segment with another: the other's corners all lie on
-// one side, further than m.  Then no edge of it meets the plane (t is beyond [0, 1] by at least m over the
-// edge, and m covers 1e-10 edges), and no point of the plane lies in it, not even by point_in_tri's
-// tolerance, which moves its edges out by less than m.
-__device__ __forceinline__ bool beyond_plane(const K1Side& P, int p, const K1Side& T, int t, int cap, double m) {
-    const double nx = P.pl[p], ny = P.pl[cap + p], nz = P.pl[2 * cap + p], d = P.pl[3 * cap + p];
-    bool above = true, below = true;
-    for (int k = 0; k < 3; ++k) {
-        const double s = nx * T.tri[(3 * k) * cap + t] + ny * T.tri[(3 * k + 1) * cap + t] + nz * T.tri[(3 * k + 2) * cap + t] + d;
-        above = above && s > m;
-        below = below && s < -m;
-    }
-    return above || below;
+// A triangle's box, rounded outward to float: min x y z, max x | max y, max z.
+__device__ __forceinline__ float4 box4(V3 a, V3 b, V3 c) {
+    return make_float4(__double2float_rd(smin3(a.x, b.x, c.x)), __double2float_rd(smin3(a.y, b.y, c.y)),
+                       __double2float_rd(smin3(a.z, b.z, c.z)), __double2float_ru(smax3(a.x, b.x, c.x)));
+}
+__device__ __forceinline__ float2 box2(V3 a, V3 b, V3 c) {
+    return make_float2(__double2float_ru(smax3(a.y, b.y, c.y)), __double2float_ru(smax3(a.z, b.z, c.z)));
+}
+__device__ __forceinline__ V3 slot_corner(const double* tri, int i, int k, int cap) {
+    return V3{tri[(3 * k) * cap + i], tri[(3 * k + 1) * cap + i], tri[(3 * k + 2) * cap + i]};
 }
 
 // |q - q0| or |q + q0|, whichever is smaller (unit quaternions; a rotation and its negative are one)
@@ -272,18 +274,26 @@ __device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned
 // CACHE: the clearance cache of a DEM step (PairArgs::cache_*), a separate instantiation so that the
 // others compile as without it.
 //
-// What bounds it: latency (loads of the soups and the survivors, barriers between a pair's phases).  The
-// overlaps of a pair are listed first and taken together: evaluating each 2,048 box tests' overlaps (about 25)
-// at once, a whole tri_tri a lane, kept two of eight warps busy through six candidates in a row.  The planes
-// leave 250 of 600 overlaps on the pair sweep.  Triangle stage on a B200: 65,536-pair sweep 24.3 -> 13.4 ms,
-// 1,500 pairs of 5,120-triangle meshes 2.66 -> 1.41, 6,000 pairs of hulls 1.41 -> 0.78, 64 mixed pairs 0.42 -> 0.23.
-// The flat test up to flat_max survivor pairs: 13.4 ms with 262,144 on the sweep, 14.7 with 8,192 (the line
-// before, when a test cost twice as much), 13.8 without a line; 1.40 against 1.58 ms on the 5,120-triangle pairs
-// (420,000 survivor pairs) with and without.
-template <bool NPX, bool CACHE>
-__global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
-    __shared__ double sh_red[2][K1_THREADS / 32];
+// What bounds it: latency (loads of the soups and the survivors, barriers between a pair's phases; ncu: 4 of 10
+// stall cycles an issue on loads, 2 on barriers, a third of the issue slots used).  The overlaps of a pair are
+// listed first and taken together: evaluating each 2,048 box tests' overlaps (about 25) at once, a whole tri_tri a
+// lane, kept two of eight warps busy through six candidates in a row.  The planes leave 250 of 600 overlaps on
+// the pair sweep.  The certificate and the culls look at a triangle's sphere (32 B) before its corners (72 B).
+// The bodies' poses are in shared memory: in registers they spilled at 80 (580 B of loads a thread, 5 % slower).
+// Triangle stage on a B200, before -> lists and planes -> spheres first and 24 warps an SM: 65,536-pair sweep 24.3
+// -> 13.4 -> 10.4 ms, 1,500 pairs of 5,120-triangle meshes 2.66 -> 1.41 -> 1.22, 6,000 pairs of hulls 1.41 -> 0.78 ->
+// 0.62, 16,384 pairs of 320-triangle meshes 1.24 -> 1.14 -> 0.72, 64 mixed pairs 0.42 -> 0.23 -> 0.25.
+// The flat test up to flat_max survivor pairs: 11.0 ms with 262,144 on the sweep, 12.3 with 8,192 (the line before,
+// when a test cost twice as much), 11.1 without a line; 1.25 against 1.36 ms on the 5,120-triangle pairs (420,000
+// survivor pairs) with and without.
+// Measured and dropped: the triangles the spheres leave listed before their corners are taken (few lanes of a warp
+// were thought to have one; neighbouring triangles are cut alike, 25 of 32 lanes were live already): 14-16 ms.
+template <bool NPX, bool CACHE, int T>
+__global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
+    __shared__ double sh_red[2][T / 32];
     __shared__ double sh_slab[3];  // hi(A.d), lo(B.d), slack of the certificate (the slab cull uses them)
+    __shared__ V3 sh_x[2];
+    __shared__ Q4 sh_q[2];
     __shared__ int sh_sep;
     __shared__ int sh_item;
     __shared__ int sh_n[2];
@@ -296,24 +306,30 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
     __shared__ unsigned long long sh_cmin, sh_gmin;
     __shared__ int sh_cbad, sh_nh;
     extern __shared__ __align__(16) unsigned char k1_dsm[];
-    // dynamic shared memory, one after the other: the hierarchical test's float boxes | keys | values | group
-    // boxes, the flat test's float boxes, the candidate points | valid bits of the triangle pairs
+    // dynamic shared memory, one after the other: the survivors' float boxes (min x y z, max x of both sides |
+    // max y, max z), the hierarchical test's float boxes | keys | values | group boxes, the candidate points |
+    // valid bits of the triangle pairs
+    float4* sm_b4 = reinterpret_cast<float4*>(k1_dsm);
+    float2* sm_b2 = reinterpret_cast<float2*>(sm_b4 + 2 * K1<T>::BCAP);
     float* sm_box = reinterpret_cast<float*>(k1_dsm);
-    uint32_t* sm_key = reinterpret_cast<uint32_t*>(sm_box + 6 * K1_HCAP);
-    int* sm_val = reinterpret_cast<int*>(sm_key + K1_HCAP);
-    float* sm_gbox = reinterpret_cast<float*>(sm_val + K1_HCAP);
+    uint32_t* sm_key = reinterpret_cast<uint32_t*>(sm_box + 6 * K1<T>::HCAP);
+    int* sm_val = reinterpret_cast<int*>(sm_key + K1<T>::HCAP);
+    float* sm_gbox = reinterpret_cast<float*>(sm_val + K1<T>::HCAP);
     const int tid = threadIdx.x;
     K1Slot S;
     char* slot = a.k1_slots + (size_t)blockIdx.x * a.k1_slot_bytes;
     carve_k1(slot, a.cap_side, a.cap_seg, &S);
     const int cap = a.cap_side;
+    const ptrdiff_t side_bytes = reinterpret_cast<char*>(S.side[1].tri) - reinterpret_cast<char*>(S.side[0].tri);
     const bool py = NPX || a.mode == 1;
     const int64_t iend = a.items ? a.item_begin + a.n_items : item_end_of(a);
 
-    for (int64_t round = 0;; ++round) {
+    // thread 0 takes the next item from the queue while this one is worked on
+    int64_t next = 0;
+    if (tid == 0) next = a.item_begin + (a.per_stage ? (int64_t)blockIdx.x : (int64_t)atomicAdd(a.queue1, 1));
+    for (;;) {
         if (tid == 0) {
-            sh_item = a.per_stage ? (int)(a.item_begin + blockIdx.x + round * gridDim.x)
-                                  : (int)(a.item_begin + atomicAdd(a.queue1, 1));
+            sh_item = next < iend ? (int)next : -1;
             sh_n[0] = sh_n[1] = 0;
             sh_nq = sh_nt = 0;
             sh_nseg = 0;
@@ -326,7 +342,8 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
         }
         __syncthreads();
         const int64_t item = sh_item;
-        if (item >= iend) break;
+        if (item < 0) break;
+        if (tid == 0) next = a.per_stage ? next + gridDim.x : a.item_begin + (int64_t)atomicAdd(a.queue1, 1);
         const int p = a.items ? a.items[item] : a.order[item];
         int chunk = 0, nchunk = 1;
         if (a.items) {
@@ -335,18 +352,22 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             nchunk = ic >> 16;
         }
         const double* ps = a.pose + 14 * (int64_t)p;
-        V3 tpos[2] = {V3{ps[0], ps[1], ps[2]}, V3{ps[7], ps[8], ps[9]}};
-        Q4 qraw[2] = {Q4{ps[3], ps[4], ps[5], ps[6]}, Q4{ps[10], ps[11], ps[12], ps[13]}};
-        Q4 qn[2];
-        for (int k = 0; k < 2; ++k) {
+        // the bodies' positions and unit quaternions, for every thread of the block (in registers they spill)
+        if (tid < 2) {
+            const double* b = ps + 7 * tid;
+            const Q4 qraw{b[3], b[4], b[5], b[6]};
+            Q4 q;
             if constexpr (NPX) {
-                double q4[4] = {qraw[k].w, qraw[k].x, qraw[k].y, qraw[k].z}, o4[4];
+                double q4[4] = {qraw.w, qraw.x, qraw.y, qraw.z}, o4[4];
                 np::quat_normalize(q4, o4);
-                qn[k] = Q4{o4[0], o4[1], o4[2], o4[3]};
+                q = Q4{o4[0], o4[1], o4[2], o4[3]};
             } else {
-                qn[k] = py ? qnormalize_py(qraw[k]) : qnormalize(qraw[k]);
+                q = py ? qnormalize_py(qraw) : qnormalize(qraw);
             }
+            sh_x[tid] = V3{b[0], b[1], b[2]};
+            sh_q[tid] = q;
         }
+        __syncthreads();
         const int mesh[2] = {a.pmesh[2 * (int64_t)p], a.pmesh[2 * (int64_t)p + 1]};
         const int64_t off[2] = {a.tri_off[mesh[0]], a.tri_off[mesh[1]]};
         const int nt[2] = {(int)(a.tri_off[mesh[0] + 1] - off[0]), (int)(a.tri_off[mesh[1] + 1] - off[1])};
@@ -356,7 +377,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
         const double R[2] = {__longlong_as_double((long long)a.mesh_R_bits[mesh[0]]),
                              __longlong_as_double((long long)a.mesh_R_bits[mesh[1]])};
         auto inf = [](V3 v) { return smax3(fabs(v.x), fabs(v.y), fabs(v.z)); };
-        const double pad = 1e-9 * (inf(tpos[0]) + inf(tpos[1]) + R[0] + R[1]);
+        const double pad = 1e-9 * (inf(sh_x[0]) + inf(sh_x[1]) + R[0] + R[1]);
         // CACHE: a pair whose entry holds (k_cache_skip) but whose near pairs meet: every triangle pair
         // that can meet is a near pair (the others are further apart than the motion), so testing those,
         // exactly as the full test does, gives the full test's segments.  The entry carries over.
@@ -369,15 +390,16 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             const uint32_t* hin = a.cache_hin + CACHE_H * (int64_t)ci;
             K1Side& DA = S.side[0];
             K1Side& DB = S.side[1];
-            for (int h = tid; h < nh; h += K1_THREADS) {
+            for (int h = tid; h < nh; h += T) {
                 const uint32_t code = hin[h];
                 const int tt[2] = {(int)(code >> 16), (int)(code & 0xffffu)};
                 bool ok = true;
+                V3 lo[2], hi[2];
                 for (int s2 = 0; s2 < 2 && ok; ++s2) {
                     K1Side& D = s2 == 0 ? DA : DB;
                     const double* v = a.tris + 9 * (off[s2] + tt[s2]);
                     V3 w[3];
-                    for (int k = 0; k < 3; ++k) w[k] = qrotate_n(qn[s2], ld3(v + 3 * k)) + tpos[s2];
+                    for (int k = 0; k < 3; ++k) w[k] = qrotate_n(sh_q[s2], ld3(v + 3 * k)) + sh_x[s2];
                     V3 n;
                     double d;
                     ok = plane_from_tri(w[0], w[1], w[2], n, d) && !(norm2(n) < 1e-30);
@@ -390,23 +412,18 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                     D.pl[1 * cap + h] = n.y;
                     D.pl[2 * cap + h] = n.z;
                     D.pl[3 * cap + h] = d;
-                    D.box[0 * cap + h] = smin3(w[0].x, w[1].x, w[2].x);
-                    D.box[1 * cap + h] = smin3(w[0].y, w[1].y, w[2].y);
-                    D.box[2 * cap + h] = smin3(w[0].z, w[1].z, w[2].z);
-                    D.box[3 * cap + h] = smax3(w[0].x, w[1].x, w[2].x);
-                    D.box[4 * cap + h] = smax3(w[0].y, w[1].y, w[2].y);
-                    D.box[5 * cap + h] = smax3(w[0].z, w[1].z, w[2].z);
+                    lo[s2] = V3{smin3(w[0].x, w[1].x, w[2].x), smin3(w[0].y, w[1].y, w[2].y), smin3(w[0].z, w[1].z, w[2].z)};
+                    hi[s2] = V3{smax3(w[0].x, w[1].x, w[2].x), smax3(w[0].y, w[1].y, w[2].y), smax3(w[0].z, w[1].z, w[2].z)};
                     D.id[h] = tt[s2];
                 }
                 if (!ok) continue;  // a triangle without a plane: the full test drops it
-                const bool sep = DA.box[3 * cap + h] < DB.box[h] || DA.box[h] > DB.box[3 * cap + h] ||
-                                 DA.box[4 * cap + h] < DB.box[cap + h] || DA.box[cap + h] > DB.box[4 * cap + h] ||
-                                 DA.box[5 * cap + h] < DB.box[2 * cap + h] || DA.box[2 * cap + h] > DB.box[5 * cap + h];
+                const bool sep = hi[0].x < lo[1].x || lo[0].x > hi[1].x || hi[0].y < lo[1].y || lo[0].y > hi[1].y ||
+                                 hi[0].z < lo[1].z || lo[0].z > hi[1].z;
                 if (!sep) S.list[1][atomicAdd(&sh_nt, 1)] = make_uint2(h, h);
             }
             double* c = a.cache_out + CACHE_W * (int64_t)p;
-            for (int k = tid; k < CACHE_W; k += K1_THREADS) c[k] = k == CACHE_SKIP ? 1.0 : e[k];
-            for (int h = tid; h < nh; h += K1_THREADS) a.cache_hout[CACHE_H * (int64_t)p + h] = hin[h];
+            for (int k = tid; k < CACHE_W; k += T) c[k] = k == CACHE_SKIP ? 1.0 : e[k];
+            for (int h = tid; h < nh; h += T) a.cache_hout[CACHE_H * (int64_t)p + h] = hin[h];
             __syncthreads();
         }
         // CACHE: the culls keep every triangle within tau more of the other body, so that each triangle
@@ -423,35 +440,64 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             bool slab = false;
             V3 dslab{0.0, 0.0, 0.0};
             if (a.mesh_infl_bits) {
-                const V3 dv = tpos[1] - tpos[0];
+                const V3 dv = sh_x[1] - sh_x[0];
                 const double dl = norm(dv);
                 const double infl = smax(__longlong_as_double((long long)a.mesh_infl_bits[mesh[0]]),
                                          __longlong_as_double((long long)a.mesh_infl_bits[mesh[1]]));
                 if (dl > 0.0 && infl < 1e300) {
                     const V3 d = dv / dl;
+                    // The extreme corner of a body is in a triangle whose sphere reaches past every centre: the
+                    // extreme centre first (32 B a triangle), then the corners of the few spheres that reach it.
+                    V3 dloc[2];
                     for (int s2 = 0; s2 < 2; ++s2) {
-                        const Q4 qc{qn[s2].w, -qn[s2].x, -qn[s2].y, -qn[s2].z};
-                        const V3 dloc = py ? qrotate_py_n(qc, d) : qrotate_n(qc, d);
-                        double e = s2 == 0 ? -__builtin_huge_val() : __builtin_huge_val();
-                        const double* tv = a.tris + 9 * off[s2];
-                        for (int q = tid; q < 3 * nt[s2]; q += K1_THREADS) {
-                            const double v = tv[3 * q] * dloc.x + tv[3 * q + 1] * dloc.y + tv[3 * q + 2] * dloc.z;
-                            e = s2 == 0 ? fmax(e, v) : fmin(e, v);
-                        }
+                        const Q4 qc{sh_q[s2].w, -sh_q[s2].x, -sh_q[s2].y, -sh_q[s2].z};
+                        dloc[s2] = py ? qrotate_py_n(qc, d) : qrotate_n(qc, d);
+                    }
+                    auto reduce = [&](int s2, double e) {  // largest of A (s2 0), smallest of B
                         for (int o = 16; o > 0; o >>= 1) {
                             const double y = __shfl_xor_sync(FULL, e, o);
                             e = s2 == 0 ? fmax(e, y) : fmin(e, y);
                         }
                         if ((tid & 31) == 0) sh_red[s2][tid >> 5] = e;
+                    };
+                    for (int s2 = 0; s2 < 2; ++s2) {
+                        double e = s2 == 0 ? -__builtin_huge_val() : __builtin_huge_val();
+                        for (int t = tid; t < nt[s2]; t += T) {
+                            const double4 sp = a.tri_sph[off[s2] + t];
+                            const double v = sp.x * dloc[s2].x + sp.y * dloc[s2].y + sp.z * dloc[s2].z;
+                            e = s2 == 0 ? fmax(e, v) : fmin(e, v);
+                        }
+                        reduce(s2, e);
+                    }
+                    __syncthreads();
+                    double best[2] = {-__builtin_huge_val(), __builtin_huge_val()};
+                    for (int w = 0; w < T / 32; ++w) {
+                        best[0] = fmax(best[0], sh_red[0][w]);
+                        best[1] = fmin(best[1], sh_red[1][w]);
+                    }
+                    __syncthreads();
+                    for (int s2 = 0; s2 < 2; ++s2) {
+                        double e = s2 == 0 ? -__builtin_huge_val() : __builtin_huge_val();
+                        for (int t = tid; t < nt[s2]; t += T) {
+                            const double4 sp = a.tri_sph[off[s2] + t];
+                            const double v = sp.x * dloc[s2].x + sp.y * dloc[s2].y + sp.z * dloc[s2].z;
+                            if (s2 == 0 ? v + sp.w + pad < best[0] : v - sp.w - pad > best[1]) continue;
+                            const double* tv = a.tris + 9 * (off[s2] + t);
+                            for (int q = 0; q < 3; ++q) {
+                                const double c = tv[3 * q] * dloc[s2].x + tv[3 * q + 1] * dloc[s2].y + tv[3 * q + 2] * dloc[s2].z;
+                                e = s2 == 0 ? fmax(e, c) : fmin(e, c);
+                            }
+                        }
+                        reduce(s2, e);
                     }
                     __syncthreads();
                     if (tid == 0) {
                         double hi = -__builtin_huge_val(), lo = __builtin_huge_val();
-                        for (int w = 0; w < K1_THREADS / 32; ++w) {
+                        for (int w = 0; w < T / 32; ++w) {
                             hi = fmax(hi, sh_red[0][w]);
                             lo = fmin(lo, sh_red[1][w]);
                         }
-                        const double hiA = dot(tpos[0], d) + hi, loB = dot(tpos[1], d) + lo;
+                        const double hiA = dot(sh_x[0], d) + hi, loB = dot(sh_x[1], d) + lo;
                         const double slack = infl * (1.0 + 1e-6) + 4.0 * pad;
                         sh_sep = (hiA + slack < loB) ? 1 : 0;
                         sh_slab[0] = hiA;
@@ -496,37 +542,41 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             double cclear = __builtin_huge_val();  // CACHE: smallest clearance of a culled triangle
             bool cbad = false;
             for (int s = 0; s < 2; ++s) {
-                const V3 other = tpos[1 - s];
-                const double lim = R[1 - s] + pad;
-                K1Side& D = S.side[s];
+                const V3 other = sh_x[1 - s];
+                const double lim = (s == 0 ? R[1] : R[0]) + pad;
+                const int64_t first = s == 0 ? off[0] : off[1];
+                // the side's arrays by their distance (an index into S would put it in local memory)
+                auto mine = [&](auto* q) { return reinterpret_cast<decltype(q)>(reinterpret_cast<char*>(q) + s * side_bytes); };
+                double* const d_tri = mine(S.side[0].tri);
+                double* const d_pl = mine(S.side[0].pl);
+                int* const d_id = mine(S.side[0].id);
                 V3 dl{0.0, 0.0, 0.0};
                 double bound = 0.0;
                 if (slab) {
-                    const Q4 qc{qn[s].w, -qn[s].x, -qn[s].y, -qn[s].z};
+                    const Q4 qc{sh_q[s].w, -sh_q[s].x, -sh_q[s].y, -sh_q[s].z};
                     dl = py ? qrotate_py_n(qc, dslab) : qrotate_n(qc, dslab);
                     // in the mesh frame: A keeps corners reaching lo(B.d) - slack, B corners below hi(A.d) + slack
-                    bound = s == 0 ? sh_slab[1] - sh_slab[2] - dot(tpos[0], dslab)
-                                   : sh_slab[0] + sh_slab[2] - dot(tpos[1], dslab);
+                    bound = s == 0 ? sh_slab[1] - sh_slab[2] - dot(sh_x[0], dslab)
+                                   : sh_slab[0] + sh_slab[2] - dot(sh_x[1], dslab);
                     if constexpr (CACHE) bound = s == 0 ? bound - tau : bound + tau;
                 }
                 const int t_lo = s == 0 ? a_lo : 0, t_hi = separated ? t_lo : (s == 0 ? a_hi : nt[1]);
-                for (int t = t_lo + tid; t < t_hi; t += K1_THREADS) {
-                    if (slab) {
-                        const double* lv = a.tris + 9 * (off[s] + t);
-                        const double p0 = lv[0] * dl.x + lv[1] * dl.y + lv[2] * dl.z;
-                        const double p1 = lv[3] * dl.x + lv[4] * dl.y + lv[5] * dl.z;
-                        const double p2 = lv[6] * dl.x + lv[7] * dl.y + lv[8] * dl.z;
-                        if (s == 0 ? (smax3(p0, p1, p2) < bound) : (smin3(p0, p1, p2) > bound)) {
-                            // CACHE: how far the triangle sits outside the slab along d
-                            if constexpr (CACHE)
-                                cclear = fmin(cclear, (s == 0 ? bound - smax3(p0, p1, p2) : smin3(p0, p1, p2) - bound) + tau);
-                            continue;
-                        }
-                    }
+                for (int t = t_lo + tid; t < t_hi; t += T) {
                     if (!a.per_stage) {
-                        double4 sp = a.tri_sph[off[s] + t];
-                        V3 c = V3{sp.x, sp.y, sp.z};
-                        V3 cw = (py ? qrotate_py_n(qn[s], c) : qrotate_n(qn[s], c)) + tpos[s];
+                        // the sphere first: wholly outside the slab, or outside the other body's cube
+                        const double4 sp = a.tri_sph[first + t];
+                        const V3 c = V3{sp.x, sp.y, sp.z};
+                        if (slab) {
+                            const double q = sp.x * dl.x + sp.y * dl.y + sp.z * dl.z;
+                            const double out = s == 0 ? bound - (q + sp.w + pad) : (q - sp.w - pad) - bound;
+                            // CACHE: how far the triangle sits outside the slab along d, at least; near the slab
+                            // its corners tell it below
+                            if (out > (CACHE ? 2.0 * tau : 0.0)) {
+                                if constexpr (CACHE) cclear = fmin(cclear, out + tau);
+                                continue;
+                            }
+                        }
+                        V3 cw = (py ? qrotate_py_n(sh_q[s], c) : qrotate_n(sh_q[s], c)) + sh_x[s];
                         double L = sp.w + lim;
                         double Lc = L;
                         if constexpr (CACHE) Lc = L + tau;
@@ -537,11 +587,23 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                             continue;
                         }
                     }
-                    const double* v = a.tris + 9 * (off[s] + t);
+                    if (slab) {
+                        const double* lv = a.tris + 9 * (first + t);
+                        const double p0 = lv[0] * dl.x + lv[1] * dl.y + lv[2] * dl.z;
+                        const double p1 = lv[3] * dl.x + lv[4] * dl.y + lv[5] * dl.z;
+                        const double p2 = lv[6] * dl.x + lv[7] * dl.y + lv[8] * dl.z;
+                        if (s == 0 ? (smax3(p0, p1, p2) < bound) : (smin3(p0, p1, p2) > bound)) {
+                            // CACHE: how far the triangle sits outside the slab along d
+                            if constexpr (CACHE)
+                                cclear = fmin(cclear, (s == 0 ? bound - smax3(p0, p1, p2) : smin3(p0, p1, p2) - bound) + tau);
+                            continue;
+                        }
+                    }
+                    const double* v = a.tris + 9 * (first + t);
                     V3 w[3];
                     for (int k = 0; k < 3; ++k) {
                         V3 lv = ld3(v + 3 * k);
-                        w[k] = (py ? qrotate_py_n(qn[s], lv) : qrotate_n(qn[s], lv)) + tpos[s];
+                        w[k] = (py ? qrotate_py_n(sh_q[s], lv) : qrotate_n(sh_q[s], lv)) + sh_x[s];
                     }
                     V3 n;
                     double d;
@@ -564,21 +626,19 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                     }
                     int i = atomicAdd(&sh_n[s], 1);
                     for (int k = 0; k < 3; ++k) {
-                        D.tri[(3 * k + 0) * cap + i] = w[k].x;
-                        D.tri[(3 * k + 1) * cap + i] = w[k].y;
-                        D.tri[(3 * k + 2) * cap + i] = w[k].z;
+                        d_tri[(3 * k + 0) * cap + i] = w[k].x;
+                        d_tri[(3 * k + 1) * cap + i] = w[k].y;
+                        d_tri[(3 * k + 2) * cap + i] = w[k].z;
                     }
-                    D.pl[0 * cap + i] = n.x;
-                    D.pl[1 * cap + i] = n.y;
-                    D.pl[2 * cap + i] = n.z;
-                    D.pl[3 * cap + i] = d;
-                    D.box[0 * cap + i] = smin3(w[0].x, w[1].x, w[2].x);
-                    D.box[1 * cap + i] = smin3(w[0].y, w[1].y, w[2].y);
-                    D.box[2 * cap + i] = smin3(w[0].z, w[1].z, w[2].z);
-                    D.box[3 * cap + i] = smax3(w[0].x, w[1].x, w[2].x);
-                    D.box[4 * cap + i] = smax3(w[0].y, w[1].y, w[2].y);
-                    D.box[5 * cap + i] = smax3(w[0].z, w[1].z, w[2].z);
-                    D.id[i] = t;
+                    d_pl[0 * cap + i] = n.x;
+                    d_pl[1 * cap + i] = n.y;
+                    d_pl[2 * cap + i] = n.z;
+                    d_pl[3 * cap + i] = d;
+                    if (i < K1<T>::BCAP) {
+                        sm_b4[s * K1<T>::BCAP + i] = box4(w[0], w[1], w[2]);
+                        sm_b2[s * K1<T>::BCAP + i] = box2(w[0], w[1], w[2]);
+                    }
+                    d_id[i] = t;
                 }
             }
             if constexpr (CACHE) {
@@ -594,17 +654,22 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
         const int64_t total = (int64_t)nA * nB;
         const K1Side& SA = S.side[0];
         const K1Side& SB = S.side[1];
-        // the survivors' exact boxes (component-major, stride cap) stay in the CTA's slot: the tests' gathers
-        // hit in L1, which staging them in shared memory (measured: slower) would take away
-        const double* bA = SA.box;
-        const double* bB = SB.box;
-        const int sA = cap, sB = cap;
         const int lcap = k1_list_cap(cap);
         const int lane = tid & 31, warp = tid >> 5;
-        // the reference's AABB reject (src/main.cpp:2130-2134), strict compares
+        // the reference's AABB reject (src/main.cpp:2130-2134), strict compares; all six at once, as a chain of
+        // short-circuits waits out a load for each
         auto meets = [&](int ia, int ib) {
-            return !((bA[3 * sA + ia] < bB[ib]) | (bA[ia] > bB[3 * sB + ib]) | (bA[4 * sA + ia] < bB[sB + ib]) |
-                     (bA[sA + ia] > bB[4 * sB + ib]) | (bA[5 * sA + ia] < bB[2 * sB + ib]) | (bA[2 * sA + ia] > bB[5 * sB + ib]));
+            V3 A[3], B[3];
+            for (int k = 0; k < 3; ++k) {
+                A[k] = slot_corner(SA.tri, ia, k, cap);
+                B[k] = slot_corner(SB.tri, ib, k, cap);
+            }
+            return !((smax3(A[0].x, A[1].x, A[2].x) < smin3(B[0].x, B[1].x, B[2].x)) |
+                     (smin3(A[0].x, A[1].x, A[2].x) > smax3(B[0].x, B[1].x, B[2].x)) |
+                     (smax3(A[0].y, A[1].y, A[2].y) < smin3(B[0].y, B[1].y, B[2].y)) |
+                     (smin3(A[0].y, A[1].y, A[2].y) > smax3(B[0].y, B[1].y, B[2].y)) |
+                     (smax3(A[0].z, A[1].z, A[2].z) < smin3(B[0].z, B[1].z, B[2].z)) |
+                     (smin3(A[0].z, A[1].z, A[2].z) > smax3(B[0].z, B[1].z, B[2].z)));
         };
         auto found = [&](int ia, int ib) {
             const int q = atomicAdd(&sh_nq, 1);
@@ -613,26 +678,33 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
         // Windows of survivor pairs, [r0, r1) of A by [c0, c1) of B: all of them at once, unless the pairs found
         // outgrow the list; then the window is halved and taken again.
         int r0 = 0, c0 = 0, rows = nA, cols = nB;
+        bool boxes = nA <= K1<T>::BCAP && nB <= K1<T>::BCAP;  // the culls' boxes are all in shared memory
+        // CACHE: survivor pairs whose boxes are less than tau apart (those that met, and so every segment,
+        // included) become the entry's near pairs, tested again at every skip; the smallest box gap of the
+        // others (the largest separation over the axes, rounded down) bounds the entry's clearance
+        float gmin = __int_as_float(0x7f800000);
+        const float near_gap = CACHE ? __double2float_ru(tau) : 0.f;
         for (;;) {
-            const int r1 = min(nA, r0 + rows), c1 = min(nB, c0 + cols);
+            const int r1 = min(nA, r0 + rows), c1 = min(nB, c0 + cols), pair = p;
             const int64_t tests = (int64_t)(r1 - r0) * (c1 - c0);
-            if (!a.per_stage && tests > a.flat_max) {
+            if (!CACHE && !a.per_stage && tests > a.flat_max) {
+                boxes = false;  // the hierarchical test uses their memory
                 // ---- hierarchical test, B's survivors a tile at a time: the tile in Morton order, outward-rounded
                 // float AABBs and 32-triangle group boxes in shared memory; one warp per A triangle rejects
                 // whole groups first.  A float reject is exact (the float box contains the double one); every
                 // float overlap is tested again below.
                 const double Rb = R[1] + pad;
-                const V3 lo = tpos[1] - V3{Rb, Rb, Rb};
+                const V3 lo = sh_x[1] - V3{Rb, Rb, Rb};
                 const double sc = 1024.0 / (2.0 * Rb);
-                for (int b0 = c0; b0 < c1; b0 += K1_HCAP) {
-                    const int nb = c1 - b0 < K1_HCAP ? c1 - b0 : K1_HCAP;
+                for (int b0 = c0; b0 < c1; b0 += K1<T>::HCAP) {
+                    const int nb = c1 - b0 < K1<T>::HCAP ? c1 - b0 : K1<T>::HCAP;
                     const int N2 = next_pow2(nb);
                     if (b0 > c0) __syncthreads();
-                    for (int i = tid; i < N2; i += K1_THREADS) {
+                    for (int i = tid; i < N2; i += T) {
                         if (i < nb) {
-                            const double* T = SB.tri + b0 + i;
-                            V3 c{T[0] + T[3 * cap] + T[6 * cap], T[cap] + T[4 * cap] + T[7 * cap],
-                                 T[2 * cap] + T[5 * cap] + T[8 * cap]};
+                            const double* t9 = SB.tri + b0 + i;
+                            V3 c{t9[0] + t9[3 * cap] + t9[6 * cap], t9[cap] + t9[4 * cap] + t9[7 * cap],
+                                 t9[2 * cap] + t9[5 * cap] + t9[8 * cap]};
                             c = c * (1.0 / 3.0);
                             sm_key[i] = morton3((c.x - lo.x) * sc, (c.y - lo.y) * sc, (c.z - lo.z) * sc);
                             sm_val[i] = b0 + i;
@@ -644,7 +716,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                     __syncthreads();
                     for (int kk2 = 2; kk2 <= N2; kk2 <<= 1)
                         for (int j = kk2 >> 1; j > 0; j >>= 1) {
-                            for (int i = tid; i < N2; i += K1_THREADS) {
+                            for (int i = tid; i < N2; i += T) {
                                 int ixj = i ^ j;
                                 if (ixj > i) {
                                     bool up = (i & kk2) == 0;
@@ -660,83 +732,101 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                             }
                             __syncthreads();
                         }
-                    for (int m = tid; m < nb; m += K1_THREADS) {
-                        int ib = sm_val[m];
-                        for (int k = 0; k < 3; ++k) sm_box[k * K1_HCAP + m] = __double2float_rd(bB[k * sB + ib]);
-                        for (int k = 3; k < 6; ++k) sm_box[k * K1_HCAP + m] = __double2float_ru(bB[k * sB + ib]);
+                    for (int m = tid; m < nb; m += T) {
+                        const int ib = sm_val[m];
+                        const V3 t0 = slot_corner(SB.tri, ib, 0, cap), t1 = slot_corner(SB.tri, ib, 1, cap),
+                                 t2 = slot_corner(SB.tri, ib, 2, cap);
+                        const float4 b4 = box4(t0, t1, t2);
+                        const float2 b2 = box2(t0, t1, t2);
+                        const float b6[6] = {b4.x, b4.y, b4.z, b4.w, b2.x, b2.y};
+                        for (int k = 0; k < 6; ++k) sm_box[k * K1<T>::HCAP + m] = b6[k];
                     }
                     __syncthreads();
                     const int ng = (nb + 31) >> 5;
-                    for (int g = warp; g < ng; g += K1_THREADS / 32) {
+                    for (int g = warp; g < ng; g += T / 32) {
                         int m = g * 32 + lane;
                         float v[6];
-                        for (int k = 0; k < 3; ++k) v[k] = m < nb ? sm_box[k * K1_HCAP + m] : __int_as_float(0x7f800000);
-                        for (int k = 3; k < 6; ++k) v[k] = m < nb ? sm_box[k * K1_HCAP + m] : -__int_as_float(0x7f800000);
+                        for (int k = 0; k < 3; ++k) v[k] = m < nb ? sm_box[k * K1<T>::HCAP + m] : __int_as_float(0x7f800000);
+                        for (int k = 3; k < 6; ++k) v[k] = m < nb ? sm_box[k * K1<T>::HCAP + m] : -__int_as_float(0x7f800000);
                         for (int o = 16; o > 0; o >>= 1) {
                             for (int k = 0; k < 3; ++k) v[k] = fminf(v[k], __shfl_xor_sync(FULL, v[k], o));
                             for (int k = 3; k < 6; ++k) v[k] = fmaxf(v[k], __shfl_xor_sync(FULL, v[k], o));
                         }
-                        if (lane < 6) sm_gbox[lane * (K1_HCAP / 32) + g] = v[lane];
+                        if (lane < 6) sm_gbox[lane * (K1<T>::HCAP / 32) + g] = v[lane];
                     }
                     __syncthreads();
-                    static_assert(K1_HCAP <= 32 * 32, "a tile's groups are one to a lane");
-                    for (int ia = r0 + warp; ia < r1; ia += K1_THREADS / 32) {
-                        float fa[6];
-                        for (int k = 0; k < 3; ++k) fa[k] = __double2float_rd(bA[k * sA + ia]);
-                        for (int k = 3; k < 6; ++k) fa[k] = __double2float_ru(bA[k * sA + ia]);
+                    static_assert(K1<T>::HCAP <= 32 * 32, "a tile's groups are one to a lane");
+                    for (int ia = r0 + warp; ia < r1; ia += T / 32) {
+                        const V3 t0 = slot_corner(SA.tri, ia, 0, cap), t1 = slot_corner(SA.tri, ia, 1, cap),
+                                 t2 = slot_corner(SA.tri, ia, 2, cap);
+                        const float4 b4 = box4(t0, t1, t2);
+                        const float2 b2 = box2(t0, t1, t2);
+                        const float fa[6] = {b4.x, b4.y, b4.z, b4.w, b2.x, b2.y};
                         // all six compares at once: a chain of short-circuits waits out a load for each
                         auto apart = [&](const float* B, int st) {
                             return bool((fa[3] < B[0]) | (fa[0] > B[3 * st]) | (fa[4] < B[st]) | (fa[1] > B[4 * st]) |
                                         (fa[5] < B[2 * st]) | (fa[2] > B[5 * st]));
                         };
-                        unsigned gbal = __ballot_sync(FULL, lane < ng && !apart(sm_gbox + lane, K1_HCAP / 32));
+                        unsigned gbal = __ballot_sync(FULL, lane < ng && !apart(sm_gbox + lane, K1<T>::HCAP / 32));
                         while (gbal) {
                             const int m = (__ffs(gbal) - 1) * 32 + lane;
                             gbal &= gbal - 1u;
-                            if (m < nb && !apart(sm_box + m, K1_HCAP)) found(ia, sm_val[m]);
-                        }
-                    }
-                }
-            } else if (!a.per_stage && tests > 0) {
-                // ---- flat test: A's boxes, rounded outward to float, in shared memory (read by every lane at
-                // once), 32 of B's in a warp's lanes; a float overlap is tested again below
-                float4* bx = reinterpret_cast<float4*>(sm_box);
-                for (int a0 = r0; a0 < r1; a0 += K1_ATILE) {
-                    const int na = r1 - a0 < K1_ATILE ? r1 - a0 : K1_ATILE;
-                    if (a0 > r0) __syncthreads();
-                    for (int i = tid; i < na; i += K1_THREADS) {
-                        const double* b = bA + a0 + i;
-                        bx[2 * i] = make_float4(__double2float_rd(b[0]), __double2float_rd(b[sA]),
-                                                __double2float_rd(b[2 * sA]), __double2float_ru(b[3 * sA]));
-                        bx[2 * i + 1] = make_float4(__double2float_ru(b[4 * sA]), __double2float_ru(b[5 * sA]), 0.f, 0.f);
-                    }
-                    __syncthreads();
-                    // a warp's unit: 32 of A against 32 of B
-                    const int ua = (na + 31) >> 5, ub = (c1 - c0 + 31) >> 5;
-                    for (int u = warp; u < ua * ub; u += K1_THREADS / 32) {
-                        const int ib = c0 + (u % ub) * 32 + lane;
-                        const double* b = bB + (ib < c1 ? ib : c1 - 1);
-                        float x0 = __double2float_rd(b[0]), y0 = __double2float_rd(b[sB]), z0 = __double2float_rd(b[2 * sB]);
-                        float x1 = __double2float_ru(b[3 * sB]), y1 = __double2float_ru(b[4 * sB]),
-                              z1 = __double2float_ru(b[5 * sB]);
-                        if (ib >= c1) x0 = __int_as_float(0x7f800000), x1 = -x0;  // no box meets it
-                        const int i0 = (u / ub) * 32, i1 = i0 + 32 < na ? i0 + 32 : na;
-#pragma unroll 4
-                        for (int i = i0; i < i1; ++i) {
-                            const float4 p = bx[2 * i];
-                            const float2 q = *reinterpret_cast<const float2*>(bx + 2 * i + 1);
-                            // all six compares at once: a chain of short-circuits branches after each
-                            const bool apart = (p.w < x0) | (p.x > x1) | (q.x < y0) | (p.y > y1) | (q.y < z0) | (p.z > z1);
-                            if (!apart) found(a0 + i, ib);
+                            if (m < nb && !apart(sm_box + m, K1<T>::HCAP)) found(ia, sm_val[m]);
                         }
                     }
                 }
             } else {
-                // the plain per-stage form: every pair given the reference's strict FP64 test
-                for (int64_t kk = tid; kk < tests; kk += K1_THREADS) {
-                    const int ia = r0 + (int)(kk / (c1 - c0)), ib = c0 + (int)(kk % (c1 - c0));
-                    if (meets(ia, ib)) found(ia, ib);
-                }
+                // ---- flat test: a warp's unit is 32 of A (read by every lane at once) against 32 of B (a lane
+                // each), on float boxes; an overlap is tested again below
+                for (int a0 = r0; a0 < r1; a0 += K1<T>::BCAP)
+                    for (int b0 = c0; b0 < c1; b0 += K1<T>::BCAP) {
+                        const int na = min(K1<T>::BCAP, r1 - a0), nb = min(K1<T>::BCAP, c1 - b0);
+                        if (!boxes) {
+                            // a tile's boxes from the slot
+                            __syncthreads();
+                            for (int i = tid; i < na + nb; i += T) {
+                                const bool sb = i >= na;
+                                const double* tt9 = sb ? SB.tri : SA.tri;
+                                const int j = sb ? b0 + i - na : a0 + i, o = sb ? K1<T>::BCAP + i - na : i;
+                                const V3 t0 = slot_corner(tt9, j, 0, cap), t1 = slot_corner(tt9, j, 1, cap), t2 = slot_corner(tt9, j, 2, cap);
+                                sm_b4[o] = box4(t0, t1, t2);
+                                sm_b2[o] = box2(t0, t1, t2);
+                            }
+                            __syncthreads();
+                        }
+                        const int ua = (na + 31) >> 5, ub = (nb + 31) >> 5;
+                        for (int u = warp; u < ua * ub; u += T / 32) {
+                            const int ob = (u % ub) * 32 + lane;
+                            const bool live = ob < nb;
+                            const float4 b4 = sm_b4[K1<T>::BCAP + (live ? ob : 0)];
+                            const float2 b2 = sm_b2[K1<T>::BCAP + (live ? ob : 0)];
+                            const int i0 = (u / ub) * 32, i1 = min(i0 + 32, na);
+#pragma unroll 4
+                            for (int i = i0; i < i1; ++i) {
+                                const float4 p = sm_b4[i];
+                                const float2 q = sm_b2[i];
+                                if constexpr (CACHE) {
+                                    const float gap = fmaxf(fmaxf(fmaxf(__fsub_rd(b4.x, p.w), __fsub_rd(p.x, b4.w)),
+                                                                  fmaxf(__fsub_rd(b4.y, q.x), __fsub_rd(p.y, b2.x))),
+                                                            fmaxf(__fsub_rd(b4.z, q.y), __fsub_rd(p.z, b2.y)));
+                                    if (live & !(gap >= near_gap)) {
+                                        const int ta = SA.id[a0 + i], tb = SB.id[b0 + ob];
+                                        const int h = atomicAdd(&sh_nh, 1);
+                                        if (ta < 65536 && tb < 65536 && h < CACHE_H)
+                                            a.cache_hout[CACHE_H * (int64_t)pair + h] = (uint32_t)ta << 16 | (uint32_t)tb;
+                                        else
+                                            sh_cbad = 1;
+                                        if (!(gap > 0.f)) found(a0 + i, b0 + ob);
+                                    } else if (live) {
+                                        gmin = fminf(gmin, gap);
+                                    }
+                                } else {
+                                    const bool apart = (p.w < b4.x) | (p.x > b4.w) | (q.x < b4.y) | (p.y > b2.x) | (q.y < b4.z) | (p.z > b2.y);
+                                    if (live & !apart) found(a0 + i, b0 + ob);
+                                }
+                            }
+                        }
+                    }
             }
             __syncthreads();
             const int nq = sh_nq;
@@ -744,18 +834,26 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                 if (rows > 1) rows = (rows + 1) >> 1;
                 else cols = (cols + 1) >> 1;
                 __syncthreads();
-                if (tid == 0) sh_nq = 0;
+                if (tid == 0) {
+                    sh_nq = 0;
+                    if constexpr (CACHE) sh_cbad = 1;  // its near pairs are listed already
+                }
                 __syncthreads();
                 continue;
             }
             // ---- the listed pairs: the reference's box test, then the planes
-            for (int q = tid; q < nq; q += K1_THREADS) {
+            for (int q = tid; q < nq; q += T) {
                 const uint2 e = S.list[0][q];
                 if (!meets(e.x, e.y)) continue;
                 if (a.tri_infl) {
                     const double more = 8.0 * pad;
-                    const bool far0 = beyond_plane(SB, e.y, SA, e.x, cap, a.tri_infl[off[0] + SA.id[e.x]] + more);
-                    const bool far1 = beyond_plane(SA, e.x, SB, e.y, cap, a.tri_infl[off[1] + SB.id[e.y]] + more);
+                    auto beyond = [&](const K1Side& P, int i, const K1Side& U, int j, double m) {
+                        return beyond_plane(V3{P.pl[i], P.pl[cap + i], P.pl[2 * cap + i]}, P.pl[3 * cap + i],
+                                            slot_corner(U.tri, j, 0, cap), slot_corner(U.tri, j, 1, cap),
+                                            slot_corner(U.tri, j, 2, cap), m);
+                    };
+                    const bool far0 = beyond(SB, e.y, SA, e.x, a.tri_infl[off[0] + SA.id[e.x]] + more);
+                    const bool far1 = beyond(SA, e.x, SB, e.y, a.tri_infl[off[1] + SB.id[e.y]] + more);
                     if (far0 | far1) continue;
                 }
                 S.list[1][atomicAdd(&sh_nt, 1)] = e;
@@ -766,20 +864,20 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
             // warps waiting on six candidates in a row.)
             {
                 const int nt2 = sh_nt;
-                double* cut = reinterpret_cast<double*>(k1_dsm);  // candidate c, coordinate k of pair j: (3c + k) K1_JOIN + j
-                unsigned* valid = reinterpret_cast<unsigned*>(cut + 18 * K1_JOIN);
-                for (int q0 = 0; q0 < nt2; q0 += K1_JOIN) {
-                    const int nj = nt2 - q0 < K1_JOIN ? nt2 - q0 : K1_JOIN;
+                double* cut = reinterpret_cast<double*>(k1_dsm);  // candidate c, coordinate k of pair j: (3c + k) K1<T>::JOIN + j
+                unsigned* valid = reinterpret_cast<unsigned*>(cut + 18 * K1<T>::JOIN);
+                for (int q0 = 0; q0 < nt2; q0 += K1<T>::JOIN) {
+                    const int nj = nt2 - q0 < K1<T>::JOIN ? nt2 - q0 : K1<T>::JOIN;
                     __syncthreads();
-                    for (int j = tid; j < nj; j += K1_THREADS) valid[j] = 0u;
+                    for (int j = tid; j < nj; j += T) valid[j] = 0u;
                     __syncthreads();
-                    for (int x = tid; x < 6 * nj; x += K1_THREADS) {
+                    for (int x = tid; x < 6 * nj; x += T) {
                         const int j = x / 6, c = x - 6 * j;
                         const uint2 e = S.list[1][q0 + j];
                         const bool sb = c >= 3;  // an edge of B against A's plane
                         const int i = sb ? c - 3 : c, i2 = i == 2 ? 0 : i + 1;
                         const double* E = (sb ? S.side[1].tri + e.y : S.side[0].tri + e.x);
-                        const double* T = (sb ? S.side[0].tri + e.x : S.side[1].tri + e.y);
+                        const double* U = (sb ? S.side[0].tri + e.x : S.side[1].tri + e.y);
                         const double* P = (sb ? S.side[0].pl + e.x : S.side[1].pl + e.y);
                         auto corner = [&](const double* t, int k) { return V3{t[3 * k * cap], t[(3 * k + 1) * cap], t[(3 * k + 2) * cap]}; };
                         const V3 n{P[0], P[cap], P[2 * cap]};
@@ -787,20 +885,20 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                         V3 o;
                         bool ok;
                         if constexpr (NPX) {
-                            const V3 t3[3] = {corner(T, 0), corner(T, 1), corner(T, 2)};
+                            const V3 t3[3] = {corner(U, 0), corner(U, 1), corner(U, 2)};
                             ok = np::tri_cut(&p0.x, &p1.x, &t3[0].x, &n.x, P[3 * cap], &o.x);
                         } else {
-                            ok = tri_cut(p0, p1, corner(T, 0), corner(T, 1), corner(T, 2), n, P[3 * cap], o);
+                            ok = tri_cut(p0, p1, corner(U, 0), corner(U, 1), corner(U, 2), n, P[3 * cap], o);
                         }
                         if (ok) {
-                            cut[(3 * c) * K1_JOIN + j] = o.x;
-                            cut[(3 * c + 1) * K1_JOIN + j] = o.y;
-                            cut[(3 * c + 2) * K1_JOIN + j] = o.z;
+                            cut[(3 * c) * K1<T>::JOIN + j] = o.x;
+                            cut[(3 * c + 1) * K1<T>::JOIN + j] = o.y;
+                            cut[(3 * c + 2) * K1<T>::JOIN + j] = o.z;
                             atomicOr(valid + j, 1u << c);
                         }
                     }
                     __syncthreads();
-                    for (int j = tid; j < nj; j += K1_THREADS) {
+                    for (int j = tid; j < nj; j += T) {
                         const unsigned v = valid[j];
                         if (__popc(v) < 2) continue;
                         const uint2 e = S.list[1][q0 + j];
@@ -811,12 +909,12 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                         bool hit;
                         if constexpr (NPX) {
                             auto pt = [&](int c, double* p) {
-                                for (int k = 0; k < 3; ++k) p[k] = cut[(3 * c + k) * K1_JOIN + j];
+                                for (int k = 0; k < 3; ++k) p[k] = cut[(3 * c + k) * K1<T>::JOIN + j];
                             };
                             hit = np::tri_join(&na.x, &nb.x, v, pt, &o0.x, &o1.x);
                         } else {
                             auto pt = [&](int c) {
-                                return V3{cut[(3 * c) * K1_JOIN + j], cut[(3 * c + 1) * K1_JOIN + j], cut[(3 * c + 2) * K1_JOIN + j]};
+                                return V3{cut[(3 * c) * K1<T>::JOIN + j], cut[(3 * c + 1) * K1<T>::JOIN + j], cut[(3 * c + 2) * K1<T>::JOIN + j]};
                             };
                             hit = tri_join(na, nb, v, pt, o0, o1, c0, c1);
                         }
@@ -834,6 +932,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                 }
                 __syncthreads();
             }
+            boxes = false;  // the candidate points used their memory
             c0 = c1;
             if (c0 >= nB) {
                 c0 = 0;
@@ -845,45 +944,22 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
         }
         if constexpr (CACHE) {
             if (!near_only) {
-                // the pair's clearance: none with a triangle without a plane.  Survivor pairs whose boxes are
-                // less than tau apart (those that met, and so every segment, included) become the entry's near pairs,
-                // tested again at every skip; the clearance is the smallest of the culled triangles' and of
-                // the other pairs' box gaps (the largest separation over the axes), at least tau
+                // the pair's clearance, at least tau: the smallest of the culled triangles' and of the far box gaps;
+                // none with a triangle without a plane or too many near pairs
                 __syncthreads();
-                const bool ok = sh_cbad == 0 && !separated;
-                uint32_t* hout = a.cache_hout + CACHE_H * (int64_t)p;
-                if (ok && nA > 0 && nB > 0) {
-                    double g = __builtin_huge_val();
-                    for (int64_t q = tid; q < total; q += K1_THREADS) {
-                        const int ia = (int)(q / nB), ib = (int)(q - (int64_t)ia * nB);
-                        double gq = -__builtin_huge_val();
-                        for (int k = 0; k < 3; ++k) {
-                            gq = fmax(gq, bB[k * sB + ib] - bA[(3 + k) * sA + ia]);
-                            gq = fmax(gq, bA[k * sA + ia] - bB[(3 + k) * sB + ib]);
-                        }
-                        if (gq < tau) {
-                            const int ta = SA.id[ia], tb = SB.id[ib];
-                            const int h = atomicAdd(&sh_nh, 1);
-                            if (ta < 65536 && tb < 65536 && h < CACHE_H) hout[h] = (uint32_t)ta << 16 | (uint32_t)tb;
-                            else sh_cbad = 1;
-                        } else {
-                            g = fmin(g, gq);
-                        }
-                    }
-                    if (g < __builtin_huge_val()) atomicMin(&sh_gmin, dbits(g));
-                }
+                if (gmin < __int_as_float(0x7f800000)) atomicMin(&sh_gmin, dbits((double)gmin));
                 __syncthreads();
                 double* c = a.cache_out + CACHE_W * (int64_t)p;
                 if (tid == 0) {
                     const double m = fmin(__longlong_as_double((long long)sh_cmin), __longlong_as_double((long long)sh_gmin));
-                    c[0] = (ok && sh_cbad == 0 && m > 0.0) ? m : -1.0;
+                    c[0] = (sh_cbad == 0 && m > 0.0) ? m : -1.0;
                 }
                 if (tid >= 1 && tid <= 14) c[tid] = ps[tid - 1];
                 if (tid == CACHE_SKIP) c[CACHE_SKIP] = 0.0;
                 if (tid == CACHE_NH) c[CACHE_NH] = (double)(sh_nh < CACHE_H ? sh_nh : CACHE_H);
                 if (tid > CACHE_NH && tid < CACHE_W) c[tid] = 0.0;
             }
-                }
+        }
         int ns = sh_nseg;
         int status = 0;
         if (ns > a.cap_seg) {
@@ -895,7 +971,7 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
         const unsigned long long sbase = sh_base;
         if (sbase + (unsigned long long)ns <= (unsigned long long)a.seg_cap) {
             // order by (ta, tb): the reference emits segments in that lexicographic order
-            for (int i = tid; i < ns; i += K1_THREADS) {
+            for (int i = tid; i < ns; i += T) {
                 uint64_t ki = S.key[i];
                 int r = 0;
                 for (int j = 0; j < ns; ++j) r += (S.key[j] < ki);
@@ -977,10 +1053,10 @@ __global__ __launch_bounds__(K1_THREADS, 2) void k_segments(PairArgs a) {
                 const long long src = __ldcg(a.chunk_seg_off + first + c);
                 const long long nc = __ldcg(a.chunk_nseg + first + c);
                 const long long take = nc < keep - run ? nc : keep - run;
-                for (long long q = tid; q < 6 * take; q += K1_THREADS)
+                for (long long q = tid; q < 6 * take; q += T)
                     a.seg[6 * (fb + run) + q] = __ldcg(a.seg + 6 * src + q);
                 if (a.seg_tri) {
-                    for (long long q = tid; q < 2 * take; q += K1_THREADS) {
+                    for (long long q = tid; q < 2 * take; q += T) {
                         a.seg_tri[2 * (fb + run) + q] = __ldcg(a.seg_tri + 2 * src + q);
                         a.seg_cand[2 * (fb + run) + q] = a.seg_cand[2 * src + q];
                     }
@@ -1086,25 +1162,26 @@ void launch_cache_skip(const PairArgs& a, int grid, cudaStream_t s) {
     if (grid > 0) k_cache_skip<<<grid, 256, 0, s>>>(a);
 }
 
+namespace {
+template <bool NPX, bool CACHE, int T>
+void launch_k1(const PairArgs& a, int grid, cudaStream_t s) {
+    auto k = k_segments<NPX, CACHE, T>;
+    // per device and cheap: set it on every launch
+    // shared memory for the resident CTAs and the rest of the SM's 256 KB as L1 (the survivors' gathers hit
+    // there): the carveout, in percent of the largest shared memory, of dynamic + static + 1 KB each
+    const int carve = (int)((100 * K1<T>::RESIDENT * (K1<T>::BYTES + 2048) + 233471) / 233472);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K1<T>::BYTES);
+    cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+    k<<<grid, T, K1<T>::BYTES, s>>>(a);
+}
+}  // namespace
+
 void launch_segments(const PairArgs& a, int grid, cudaStream_t s) {
     if (grid <= 0) return;
-    // per device and cheap: set it on every launch
-    // shared memory for two CTAs per SM and the rest of the SM's 256 KB as L1 (the survivors' gathers hit
-    // there): the carveout, in percent of the largest shared memory, that holds 2 x (dynamic + static + 1 KB)
-    const int carve = (int)((200 * (K1_DSMEM + 2048) + 233471) / 233472);
-    if (a.mode == 2) {
-        cudaFuncSetAttribute(k_segments<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K1_DSMEM);
-        cudaFuncSetAttribute(k_segments<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-        k_segments<true, false><<<grid, K1_THREADS, K1_DSMEM, s>>>(a);
-    } else if (a.cache_out && !a.items && a.mode == 0) {
-        cudaFuncSetAttribute(k_segments<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K1_DSMEM);
-        cudaFuncSetAttribute(k_segments<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-        k_segments<false, true><<<grid, K1_THREADS, K1_DSMEM, s>>>(a);
-    } else {
-        cudaFuncSetAttribute(k_segments<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K1_DSMEM);
-        cudaFuncSetAttribute(k_segments<false, false>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-        k_segments<false, false><<<grid, K1_THREADS, K1_DSMEM, s>>>(a);
-    }
+    const bool small = a.k1_threads == 128;
+    if (a.mode == 2) launch_k1<true, false, 256>(a, grid, s);
+    else if (a.cache_out && !a.items && a.mode == 0) small ? launch_k1<false, true, 128>(a, grid, s) : launch_k1<false, true, 256>(a, grid, s);
+    else small ? launch_k1<false, false, 128>(a, grid, s) : launch_k1<false, false, 256>(a, grid, s);
 }
 
 // --------------------------------------------------------------------------------------------- stage 2

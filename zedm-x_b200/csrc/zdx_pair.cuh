@@ -78,6 +78,7 @@ struct PairArgs {
     int32_t* chunk_nseg;
     int32_t* chunk_status;
     int64_t n_items;
+    int k1_threads;  // threads of a CTA, 128 or 256 (triangle_threads)
     char* k1_slots;
     size_t k1_slot_bytes;
     double* seg;  // arena: 6 doubles per segment
@@ -182,6 +183,10 @@ constexpr int TEAM_COUNTS = 16;
 int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s);
 // Bytes of one triangle-stage slot.
 size_t tritest_slot_bytes(int cap_side, int cap_seg);
+// Threads of a triangle-stage CTA for a batch (PairArgs::k1_threads), and the CTAs an SM runs for the tuning value
+// tri_ctas_per_sm (1, or 2: as many as fit).
+int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode);
+int triangle_ctas(int knob, int threads);
 
 void launch_mesh_prep(const PairArgs& a, int64_t total_tris, cudaStream_t s);
 void launch_cost_order(const PairArgs& a, int32_t* order, int* buckets, cudaStream_t s);

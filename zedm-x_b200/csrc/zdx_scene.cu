@@ -1556,7 +1556,9 @@ static int graph_alloc(zdx_ctx* ctx, Scene& s) {
     CKS(G.pair_i32.ensure(sizeof(int32_t) * 6 * P1));
     CKS(G.counters.ensure(sizeof(unsigned long long) * 16 + sizeof(int) * TEAM_COUNTS));
     CKS(G.tm_lists.ensure(sizeof(int32_t) * (TEAM_CLASSES + 1) * P1));
-    G.k1_grid = (int)std::min<int64_t>(P1, (int64_t)ctx->num_sms * ctx->tune.tri_ctas_per_sm);
+    // a small scene has few pairs, whatever its capacity
+    G.k1_threads = s.np < kCacheMinParticles ? 256 : triangle_threads(max_ntri, (int64_t)P1, ctx->num_sms, ZDX_MODE_ZDEM);
+    G.k1_grid = (int)std::min<int64_t>(P1, (int64_t)ctx->num_sms * triangle_ctas(ctx->tune.tri_ctas_per_sm, G.k1_threads));
     CKS(G.k1_slots.ensure(tritest_slot_bytes(max_ntri, G.cap_seg) * (size_t)G.k1_grid));
     CKS(G.seg_arena.ensure(sizeof(double) * 6 * (size_t)std::max<int64_t>(G.segcap, 1)));
     const size_t slot = rebuild_slot_bytes(G.cap_seg);
@@ -1664,6 +1666,7 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         a.cap_side = max_ntri;
         a.cap_seg = G.cap_seg;
         a.flat_max = ctx->tune.flat_max;
+        a.k1_threads = G.k1_threads;
         const size_t P1 = (size_t)std::max<int64_t>(G.pcap, 1);
         int64_t* pi64 = as<int64_t>(G.pair_i64);
         int32_t* pi32 = as<int32_t>(G.pair_i32);

@@ -107,7 +107,7 @@ struct GraphStep {
     bool ff_next = true;       // a small scene's next call tries free flight first (its last step had no candidate)
     cudaGraphExec_t exec = nullptr;
     int64_t pcap = 0, ccap = 0, wcap = 0, segcap = 0;
-    int cap_seg = 0, k2_warps = 0, k1_grid = 0, wall_warps = 0, max_wtri = 1, kernels_per_step = 0;
+    int cap_seg = 0, k2_warps = 0, k1_grid = 0, k1_threads = 256, wall_warps = 0, max_wtri = 1, kernels_per_step = 0;
     int64_t spts = 0;
     uint32_t T = 1;
     int bits = 0, pbits = 1;

@@ -426,8 +426,13 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
     TeamShared& sh = *tm.sh;
     const bool py = NPX || a.mode == 1;
     const bool split = a.split != 0;
+    // Lanes that leave an item early wait for the others of their warp: left to themselves they go on to their
+    // next items apart (the trip count is the same for every lane, so that all of them get to the wait).
     auto each = [&](int count, auto&& f) {
-        for (int i = tm.t; i < count; i += Team::T) f(i);
+        for (int b = 0; b < count; b += Team::T) {
+            if (b + tm.t < count) f(b + tm.t);
+            tm.warp_sync();
+        }
     };
     each(np, [&](int k) {
         TeamPair& P = sh.pr[k];
@@ -521,17 +526,24 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
             const int b = sh.first[k], e = sh.first[k + 1];
             const int i = b + 32 * ti + (q & 31), j0 = b + 32 * (ti + task - first), j1 = j0 + 32 < e ? j0 + 32 : e;
             const float4 p0 = bx[2 * (i < e ? i : e - 1)], p1 = bx[2 * (i < e ? i : e - 1) + 1];
+            // four at a time, their hits afterwards: the loads of one do not wait for the list of another
+            for (int j = j0; j < j1; j += 4) {
+                unsigned hit = 0;
 #if defined(__CUDA_ARCH__)
-#pragma unroll 4
+#pragma unroll
 #endif
-            for (int j = j0; j < j1; ++j) {
-                const float4 o0 = bx[2 * j], o1 = bx[2 * j + 1];
-                // all six compares at once: a chain of short-circuits waits out a load for each
-                const bool apart = (p0.w < o0.x) | (p0.x > o0.w) | (p1.x < o0.y) | (p0.y > o1.x) | (p1.y < o0.z) | (p0.z > o1.y);
-                if (!apart & (i < j) & (i < e)) {
-                    const int o = Team::add(&sh.n_list, 1);
-                    if (o < list_cap) list[o] = (uint32_t)i | (uint32_t)j << 16;
+                for (int r = 0; r < 4; ++r) {
+                    const float4 o0 = bx[2 * (j + r < j1 ? j + r : j)], o1 = bx[2 * (j + r < j1 ? j + r : j) + 1];
+                    // all six compares at once: a chain of short-circuits waits out a load for each
+                    const bool apart = (p0.w < o0.x) | (p0.x > o0.w) | (p1.x < o0.y) | (p0.y > o1.x) | (p1.y < o0.z) | (p0.z > o1.y);
+                    hit |= (!apart & (i < j + r) & (j + r < j1) & (i < e)) ? 1u << r : 0u;
                 }
+                for (int r = 0; hit; hit >>= 1, ++r) {
+                    if (!(hit & 1u)) continue;
+                    const int o = Team::add(&sh.n_list, 1);
+                    if (o < list_cap) list[o] = (uint32_t)i | (uint32_t)(j + r) << 16;
+                }
+                tm.warp_sync();  // or the lanes go on apart, each with its own rest of the tile
             }
         }
     }
