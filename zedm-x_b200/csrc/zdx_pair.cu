@@ -651,7 +651,6 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
             __syncthreads();
         }
         const int nA = near_only ? 0 : sh_n[0], nB = near_only ? 0 : sh_n[1];
-        const int64_t total = (int64_t)nA * nB;
         const K1Side& SA = S.side[0];
         const K1Side& SB = S.side[1];
         const int lcap = k1_list_cap(cap);

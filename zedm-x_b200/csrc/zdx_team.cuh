@@ -1062,7 +1062,8 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
         }
         tm.sync();
     }
-    each(ncomp, [&](int c) {
+    // one thread a component, neighbours in different warps (lanes that walk apart take turns)
+    for (int c = tm.warp() + Team::WARPS * tm.lane(); c < ncomp; c += Team::T) {
         int* vo = vord + vbase[c];
         const int nv = vbase[c + 1] - vbase[c];
         // (up to 16 std::sort is an insertion sort, which is stable; more are sorted already)
@@ -1113,7 +1114,7 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
             }
         }
         nl[c] = count;
-    });
+    }
     tm.sync();
     const int nloops = team_scan(tm, nl, ncomp);
     each(np, [&](int k) { sh.pr[k].loop0 = nl[sh.pr[k].comp0]; });
