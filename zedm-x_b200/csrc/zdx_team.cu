@@ -82,8 +82,12 @@ __global__ void __launch_bounds__(T, BLOCKS) k_rebuild_team(PairArgs a, TeamPlan
     tm.t = threadIdx.x;
     tm.sh = &sh;
     const int count = pl.counts[cls];
-    // few enough a claim that every block gets some
-    const int claim = max(1, min(TEAM_PACK, count / (2 * (int)gridDim.x)));
+    // A claim is a number of items that are `claims` apart in the list (which is sorted by cost, so that claims are
+    // alike): one claim a block where that is a few items (a pack takes the time of its longest chains, whether
+    // it holds one small pair or eight), two or more a block otherwise.
+    const int blocks = (int)gridDim.x, per = (count + blocks - 1) / blocks;
+    const int claim = max(1, min(TEAM_PACK, per <= 4 ? per : (per + 1) / 2));
+    const int claims = (count + claim - 1) / claim;
     const int32_t* list = pl.lists + cls * pl.stride;
     if (threadIdx.x == 0) sh.from = sh.to = 0;
     int again = 0, held = 0;  // pairs of a refused pack still to be taken alone
@@ -98,13 +102,14 @@ __global__ void __launch_bounds__(T, BLOCKS) k_rebuild_team(PairArgs a, TeamPlan
         } else if (threadIdx.x < 32) {
             const int lane = threadIdx.x;
             int from = sh.from, to = sh.to;
-            if (from == to) {
-                if (lane == 0) from = atomicAdd(pl.counts + 8 + cls, claim);
+            if (from >= to) {  // items from, from + claims, ... below to
+                if (lane == 0) from = atomicAdd(pl.counts + 8 + cls, 1);
                 from = __shfl_sync(0xffffffffu, from, 0);
-                to = min(count, from + claim);
+                to = from < claims ? count : from;
             }
-            const bool live = from + lane < to;
-            const int p = live ? list[from + lane] : 0;
+            const int64_t at = from + (int64_t)lane * claims;
+            const bool live = at < to;
+            const int p = live ? list[at] : 0;
             int sum = live ? a.pair_nseg[p] : 0;
             for (int d = 1; d < 32; d <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, sum, d);
@@ -115,8 +120,8 @@ __global__ void __launch_bounds__(T, BLOCKS) k_rebuild_team(PairArgs a, TeamPlan
             if (lane < np) sh.pr[lane].p = sh.claimed[lane] = p;
             if (lane == 0) {
                 sh.np = np;
-                sh.from = from + np;
-                sh.to = max(to, from + np);
+                sh.from = from + np * claims;
+                sh.to = to;
             }
         }
         tm.sync();
