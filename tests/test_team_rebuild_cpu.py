@@ -59,7 +59,7 @@ def _pairs(oracle, split, mode, tols):
 
     rng = np.random.default_rng(77)
     raw = []
-    for la, lb in ((1, 1), (1, 2), (2, 2), (1, 3), (3, 1), (2, 3), (3, 3), (1, 4), (4, 2)):
+    for la, lb in ((1, 1), (1, 2), (2, 2), (1, 3), (3, 1), (2, 3), (3, 3), (1, 4), (4, 2), (4, 4)):
         for _ in range(4 if max(la, lb) < 4 else 2):
             raw.append((synth.noised_icosphere(la, 1e-3, 0.15, rng), synth.noised_icosphere(lb, 1e-3, 0.15, rng),
                         synth.pair_poses(rng, 1, 1e-3, 0.05, 0.5)[0], f"ico {la} {lb}"))
@@ -107,12 +107,12 @@ def _check(o, k, entry, polyline):
     return n
 
 
-MODES = [(0, True), (0, False), (1, False), (2, False)]  # polyline's split search is not in the team form
+MODES = [(0, True), (0, False), (1, True), (1, False), (2, True), (2, False)]
 
 
 @pytest.mark.parametrize("mode,split", MODES)
 def test_team_rebuild_matches_oracle(team, oracle, mode, split):
-    seen = big = cut = 0
+    seen = big = cut = most = 0
     for tol, entries in _pairs(oracle, split, mode, (0.0,) if mode == 0 else (1e-6, 2e-5)).items():
         for en in entries:
             o = team([en[:4]], mode, split, tol)
@@ -120,8 +120,10 @@ def test_team_rebuild_matches_oracle(team, oracle, mode, split):
                 cut += 1
                 continue
             seen += _check(o, 0, en, mode != 0)
-            big = max(big, en[0]["nseg"])
-    assert seen > 40 and big > 100 and cut <= 2
+            big, most = max(big, en[0]["nseg"]), max(most, en[0]["ncomp"])
+    assert seen > 40 and big > 300 and cut <= 2
+    if split and mode:
+        assert most > 16  # components sorted: above 16 std::sort and Python's sort part
 
 
 @pytest.mark.parametrize("mode,split", MODES)

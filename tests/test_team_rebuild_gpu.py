@@ -27,7 +27,8 @@ def _batch():
     return lib, np.array(pm, np.int32)[order], np.concatenate(pp)[order]
 
 
-@pytest.mark.parametrize("mode,split,tol", [(0, True, 0.0), (0, False, 0.0), (1, False, 1e-6), (1, False, 3e-5), (2, False, 2e-5)])
+@pytest.mark.parametrize("mode,split,tol", [(0, True, 0.0), (0, False, 0.0), (1, False, 1e-6), (1, True, 3e-5), (2, False, 2e-5),
+                                            (2, True, 1e-6)])
 def test_teams_match_warp_form(ctx, mode, split, tol):
     from zdemx import _lib
 

@@ -612,8 +612,8 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
             CK(cudaMemsetAsync(a.pair_status, 0, sizeof(int32_t) * P1, st));
             if (a.pair_done) CK(cudaMemsetAsync(a.pair_done, 0, sizeof(int32_t) * NP, st));
         }
-        // stage 2: rebuild, by teams in shared memory; the pairs no team holds, every pair of the plain
-        // per-stage form and of polyline's split search, one warp per pair, slots sized for the largest pair
+        // stage 2: rebuild, by teams in shared memory; the pairs no team holds and every pair of the plain
+        // per-stage form one warp per pair, slots sized for the largest pair
         const int nmax = std::max(((int*)&hc[6])[0], 1);
         const size_t budget = (size_t)2 << 30;
         auto warp_form = [&](const int32_t* order, const int64_t pairs) -> int {
@@ -634,7 +634,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
         };
         const bool arena = ctx->tune.rebuild_arena != 0 && a.mode == 0 && !a.tape_stage && !a.want_pts &&
                            !a.comp_stats && !a.per_stage;
-        const bool teams = !arena && !a.per_stage && (a.mode == 0 || !a.split);
+        const bool teams = !arena && !a.per_stage;
         TeamPlan plan{};
         if (teams) {
             CK(ctx->tm_lists.ensure(sizeof(int32_t) * (TEAM_CLASSES + 1) * P1));

@@ -13,7 +13,7 @@
 
 // Left to the compiler's inlining on the device (forcing it raises the rebuild kernel's spills).
 #ifdef __CUDACC__
-#define ZDX_HD_SET __host__ __device__
+#define ZDX_HD_SET inline __host__ __device__
 #else
 #define ZDX_HD_SET inline
 #endif

@@ -28,6 +28,7 @@
 #include "zdx_math.cuh"
 #include "zdx_npmath.cuh"
 #include "zdx_pair.cuh"
+#include "zdx_pyset.cuh"
 #include "zdx_sortrep.cuh"
 
 namespace zdx {
@@ -100,6 +101,7 @@ struct DevTeam {
     }
     static __device__ __forceinline__ int add(int* p, int v) { return atomicAdd(p, v); }
     static __device__ __forceinline__ int cas(int* p, int was, int v) { return atomicCAS(p, was, v); }
+    static __device__ __forceinline__ void max(int* p, int v) { atomicMax(p, v); }
     static __device__ __forceinline__ unsigned long long take(unsigned long long* p, unsigned long long v) {
         return atomicAdd(p, v);
     }
@@ -131,6 +133,7 @@ struct HostTeam {
         *p += v;
         return o;
     }
+    static ZDX_HD void max(int* p, int v) { *p = *p < v ? v : *p; }
     static ZDX_HD int cas(int* p, int was, int v) {
         const int o = *p;
         if (o == was) *p = v;
@@ -419,13 +422,15 @@ ZDX_HD bool team_contact(V3 Sn, V3 Gn, double diag, bool py, double tol, double 
 }
 
 // The rebuild of the pairs sh.pr[0..np), each with at least one segment and status 0.  False: the pack is not
-// held here (see above).  Polyline modes take no split here (their search visits candidates in the order of a
-// Python set).
+// held here (see above).
 template <class Team, bool NPX>
 ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* sm, const int bytes) {
     TeamShared& sh = *tm.sh;
     const bool py = NPX || a.mode == 1;
     const bool split = a.split != 0;
+    // polyline.py's search visits a segment's candidates, all those with adjacent rep cells, in the order of a
+    // Python set (zdx_pyset.cuh)
+    const bool by_set = py && split;
     // Lanes that leave an item early wait for the others of their warp: left to themselves they go on to their
     // next items apart (the trip count is the same for every lane, so that all of them get to the wait).
     auto each = [&](int count, auto&& f) {
@@ -490,6 +495,8 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
         sp[i] = (unsigned char)k;
         const TeamPair& P = sh.pr[k];
         const double h = P.h;
+        // boxes that overlap wherever rep cells are adjacent, for which the set wants all
+        const double hb = by_set ? h * (1.0 + 1e-6) : h;
         const double* g = a.seg + 6 * (a.pair_seg_off[P.p] + (i - sh.first[k]));
         const V3 p0 = team_ld(g), p1 = team_ld(g + 3);
         team_st(S + 6 * i, p0);
@@ -500,9 +507,9 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
             in = team_cell(cell_of(r == 0 ? p0 : r == 1 ? p1 : (p0 + p1) * 0.5, h), P.c0, &c) && in;
             team_put(rc + 12 * i + 4 * r, c);
         }
-        bx[2 * i] = float4{team_down(smin(p0.x, p1.x) - h), team_down(smin(p0.y, p1.y) - h), team_down(smin(p0.z, p1.z) - h),
-                           team_up(smax(p0.x, p1.x) + h)};
-        bx[2 * i + 1] = float4{team_up(smax(p0.y, p1.y) + h), team_up(smax(p0.z, p1.z) + h), 0.f, 0.f};
+        bx[2 * i] = float4{team_down(smin(p0.x, p1.x) - hb), team_down(smin(p0.y, p1.y) - hb), team_down(smin(p0.z, p1.z) - hb),
+                           team_up(smax(p0.x, p1.x) + hb)};
+        bx[2 * i + 1] = float4{team_up(smax(p0.y, p1.y) + hb), team_up(smax(p0.z, p1.z) + hb), 0.f, 0.f};
         if (!in) sh.bad = 1;
     });
     tm.sync();
@@ -553,7 +560,7 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
     M.hi = bytes & ~15;  // the boxes are dead
 
     // ---- the neighbours among them: some rep cells adjacent.  Entry: i | j << 13 | walk rank of j from i
-    // << 26 | of i from j << 33 | close endpoints (bit 2 ei + ej) << 40 | DFS edge << 44.  They grow down
+    // << 26 | of i from j << 33 | close endpoints (bit 2 ei + ej) << 40 | DFS edge << 44 | boxes meet << 45.  They grow down
     // from the end of the memory.
     unsigned long long* near_top = reinterpret_cast<unsigned long long*>(sm + M.hi);
     const int near_cap = (M.hi - ((M.lo + 4 * nlist + 15) & ~15)) / 8;
@@ -562,10 +569,11 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
         const double h = sh.pr[sp[i]].h;
         const V3 a0 = team_ld(S + 6 * i), a1 = team_ld(S + 6 * i + 3), b0 = team_ld(S + 6 * j), b1 = team_ld(S + 6 * j + 3);
         // the reference's box test in FP64 (the floats only rule out)
-        if (smax(a0.x, a1.x) + h < smin(b0.x, b1.x) - h || smin(a0.x, a1.x) - h > smax(b0.x, b1.x) + h ||
-            smax(a0.y, a1.y) + h < smin(b0.y, b1.y) - h || smin(a0.y, a1.y) - h > smax(b0.y, b1.y) + h ||
-            smax(a0.z, a1.z) + h < smin(b0.z, b1.z) - h || smin(a0.z, a1.z) - h > smax(b0.z, b1.z) + h)
-            return;
+        const bool meet =
+            !(smax(a0.x, a1.x) + h < smin(b0.x, b1.x) - h || smin(a0.x, a1.x) - h > smax(b0.x, b1.x) + h ||
+              smax(a0.y, a1.y) + h < smin(b0.y, b1.y) - h || smin(a0.y, a1.y) - h > smax(b0.y, b1.y) + h ||
+              smax(a0.z, a1.z) + h < smin(b0.z, b1.z) - h || smin(a0.z, a1.z) - h > smax(b0.z, b1.z) + h);
+        if (!meet && !by_set) return;
         // smallest walk rank r * 27 + cell over the adjacent rep points, from either side
         int kij = 127, kji = 127, close = 0;
         for (int r = 0; r < 3; ++r) {
@@ -585,7 +593,8 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
         const int o = Team::add(&sh.n_near, 1);
         if (o < near_cap)
             near_top[-1 - o] = (unsigned long long)i | (unsigned long long)j << 13 | (unsigned long long)kij << 26 |
-                               (unsigned long long)kji << 33 | (unsigned long long)close << 40;
+                               (unsigned long long)kji << 33 | (unsigned long long)close << 40 |
+                               (meet ? 1ull << 45 : 0ull);
     });
     tm.sync();
     const int nnear = sh.n_near;
@@ -617,16 +626,29 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
             const int i = (int)(w & 0x1fff), j = (int)((w >> 13) & 0x1fff);
             const V3 a0 = team_ld(S + 6 * i), a1 = team_ld(S + 6 * i + 3), b0 = team_ld(S + 6 * j), b1 = team_ld(S + 6 * j + 3);
             const double tol2 = sh.pr[sp[i]].h * sh.pr[sp[i]].h;
-            const bool ij = seg_seg_dist2(a0, a1, b0, b1) <= tol2;
-            const bool ji = seg_seg_dist2(b0, b1, a0, a1) <= tol2;
-            // the search takes whichever direction it meets first: only where both agree is the component
-            // known without it
-            if (ij != ji) sh.bad = 1;
-            if (!ij) return;
-            near_top[-1 - k] = w | 1ull << 44;
-            team_unite<Team>(lab, i, j);
-            Team::add(end + i, 1);
-            Team::add(end + j, 1);
+            bool edge = false;
+            if (w >> 45 & 1) {
+                bool ij, ji;
+                if constexpr (NPX) {
+                    ij = np::seg_seg_dist2(&a0.x, &a1.x, &b0.x, &b1.x) <= tol2;
+                    ji = np::seg_seg_dist2(&b0.x, &b1.x, &a0.x, &a1.x) <= tol2;
+                } else {
+                    ij = seg_seg_dist2(a0, a1, b0, b1) <= tol2;
+                    ji = seg_seg_dist2(b0, b1, a0, a1) <= tol2;
+                }
+                // the search takes whichever direction it meets first: only where both agree is the component
+                // known without it
+                if (ij != ji) sh.bad = 1;
+                edge = ij;
+            }
+            if (edge) {
+                near_top[-1 - k] = w | 1ull << 44;
+                team_unite<Team>(lab, i, j);
+            }
+            if (edge || by_set) {
+                Team::add(end + i, 1);
+                Team::add(end + j, 1);
+            }
         });
         tm.sync();
         if (sh.bad) return false;
@@ -651,10 +673,12 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
         tm.sync();
         each(nnear, [&](int k) {
             const unsigned long long w = near_top[-1 - k];
-            if (!(w >> 44 & 1)) return;
+            const uint32_t edge = (uint32_t)(w >> 44 & 1);
+            if (!edge && !by_set) return;
             const int i = (int)(w & 0x1fff), j = (int)((w >> 13) & 0x1fff);
-            adj[Team::add(end + i, 1)] = (uint32_t)(w >> 26 & 0x7f) << 16 | (uint32_t)j;
-            adj[Team::add(end + j, 1)] = (uint32_t)(w >> 33 & 0x7f) << 16 | (uint32_t)i;
+            // walk rank << 16 | segment << 1 | DFS edge
+            adj[Team::add(end + i, 1)] = (uint32_t)(w >> 26 & 0x7f) << 16 | (uint32_t)j << 1 | edge;
+            adj[Team::add(end + j, 1)] = (uint32_t)(w >> 33 & 0x7f) << 16 | (uint32_t)i << 1 | edge;
         });
         each(n, [&](int i) { Team::add(csort + cid[root[i]], 1); });
         tm.sync();
@@ -672,7 +696,44 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
             lab[i] = e0 | (e1 - e0) << 16;  // from here the segment's list: first entry, length
         });
         tm.sync();
-        // a pair's components by size, descending, ties as std::sort leaves them (src/main.cpp:897), on packed words
+        if (by_set) {
+            // each list's edges alone, in the order of the set its candidates make when they are added in list order
+            if (tm.t == 0) sh.hits = 0;
+            tm.sync();
+            each(n, [&](int i) { Team::max(&sh.hits, (int)((uint32_t)lab[i] >> 16)); });
+            tm.sync();
+            const int most = sh.hits, words = 10 * most + 8;
+            const int left = (M.hi - M.lo) / 4 / words, lanes = left < Team::T ? left : Team::T;
+            tm.sync();
+            if (tm.t == 0) sh.hits = 0;
+            if (lanes < 1) return false;
+            int* tab = reinterpret_cast<int*>(sm + M.lo) + tm.t * words;
+            for (int b = 0; b < n; b += lanes) {
+                const int i = b + tm.t;
+                if (tm.t < lanes && i < n) {
+                    const int e0 = lab[i] & 0xffff, nc = (int)((uint32_t)lab[i] >> 16), s0 = sh.first[sp[i]];
+                    int *old = tab + 8 * most + 8, *keys = old + most;
+                    for (int q = 0; q < nc; ++q) keys[q] = ((int)(adj[e0 + q] & 0xffffu) >> 1) - s0;
+                    bool ok = true;
+                    const unsigned mask = pyset_build(keys, nc, tab, old, &ok);
+                    if (!ok) sh.bad = 1;
+                    int cnt = 0;
+                    for (unsigned x = 0; x <= mask; ++x) {
+                        if (tab[x] < 0) continue;
+                        int q = 0;
+                        while (keys[q] != tab[x]) ++q;
+                        if (adj[e0 + q] & 1u) old[cnt++] = tab[x];
+                    }
+                    for (int q = 0; q < cnt; ++q) adj[e0 + q] = (uint32_t)(old[q] + s0) << 1 | 1u;
+                    lab[i] = e0 | cnt << 16;
+                }
+                tm.warp_sync();
+            }
+            tm.sync();
+            if (sh.bad) return false;
+        }
+        // a pair's components by size, descending, ties as std::sort leaves them (src/main.cpp:897; Python's sort is
+        // stable), on packed words
         unsigned short* tmp = M.take<unsigned short>(3L * (ncomp + np));
         if (!M.ok) return false;
         for (int k = tm.warp(); k < np; k += Team::WARPS) {
@@ -680,8 +741,9 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
             for (int c = c0 + tm.lane(); c < c1; c += Team::LANES) csort[c] = (32767 - csort[c]) << 16 | c;
             tm.warp_sync();
             unsigned short* t = tmp + 3 * (c0 + k);
-            team_std_sort(tm, csort + c0, c1 - c0, t, t + (c1 - c0) + 1, t + 2 * (c1 - c0) + 2);
+            if (!py) team_std_sort(tm, csort + c0, c1 - c0, t, t + (c1 - c0) + 1, t + 2 * (c1 - c0) + 2);
             if (tm.lane() != 0) continue;
+            if (py) stable_sort_idx(csort + c0, c1 - c0, [](int x, int y) { return (x >> 16) < (y >> 16); });
             sh.pr[k].comp0 = c0;
             int run = sh.first[k];
             for (int c = c0; c < c1; ++c) {
@@ -709,7 +771,7 @@ ZDX_HD bool team_rebuild(const Team& tm, const PairArgs& a, const int np, char* 
                 const int e0 = lab[i] & 0xffff, e1 = e0 + (int)((uint32_t)lab[i] >> 16);
                 for (int x0 = e0; x0 < e1; x0 += Team::LANES) {
                     const int x = x0 + tm.lane();
-                    const int j = x < e1 ? (int)(adj[x] & 0xffffu) : 0;
+                    const int j = x < e1 ? (int)(adj[x] & 0xffffu) >> 1 : 0;
                     const bool fresh = x < e1 && !seen[j];
                     const unsigned bal = tm.ballot(fresh);
                     if (!bal) continue;
