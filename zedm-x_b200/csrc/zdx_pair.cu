@@ -1067,93 +1067,153 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
     }
 }
 
+constexpr int CSKIP_PAIRS = 16;
+
 // A clearance M found at an earlier step still holds while the vertices' displacements since then add
 // up to less than M: a vertex of body s moves by at most |x - x0| + 2 |v| |q - q0| (|R(q) v - R(q0) v| =
 // 2 sin(theta / 2) |v| <= 2 |q - q0| |v| for unit quaternions, |v| <= R).  M covers every triangle pair
 // but the entry's near pairs, which are tested again as the full test does (world corners, plane,
 // strict box compare, tri_tri).  With none of them meeting, the pair has no segment, as when the
 // separation certificate holds; otherwise k_segments tests the near pairs alone (their segments are
-// all the pair has), or in full when the motion exceeds M.  Warp per pair, lanes over the near pairs.
-// (Three blocks of 256 per SM: 80 registers with some spills, 0.8 % faster on the pour than 128.)
+// all the pair has), or in full when the motion exceeds M.
+//
+// A warp takes its share of the pairs, up to CSKIP_PAIRS consecutive ones, together: lanes over the pairs for the
+// motion, then over all their near pairs, one behind the other, until one of a pair's meets.  Bound: FP64
+// instructions (issue 0.49, a third of the FP64 pipe's cycles) and the near pairs' corners, which L1 and L2 hold.
+// With a warp per pair the motion (four normalised quaternions in a row) ran on every lane alike and a pair's last
+// near pairs left lanes idle: 87,000 pairs of the pour, 0.40 ms.  Shared out: 0.228 ms.
+struct CacheSkipWarp {
+    double pose[CSKIP_PAIRS][15];  // positions and unit quaternions of A and B (one word of padding: banks)
+    int64_t off[CSKIP_PAIRS][2];   // first triangles
+    int ci[CSKIP_PAIRS];
+    unsigned meet;  // bit per pair: a near pair meets
+};
+
 __global__ __launch_bounds__(256, 3) void k_cache_skip(PairArgs a) {
+    __shared__ CacheSkipWarp sh[8];
+    CacheSkipWarp& W = sh[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     const int64_t n = pairs_of(a);
-    for (int64_t p = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); p < n; p += warps) {
-        const int ci = a.cache_idx[p];
-        int flag = 0;
+    const int64_t share = (n + warps - 1) / warps;
+    const int G = share < 1 ? 1 : share > CSKIP_PAIRS ? CSKIP_PAIRS : (int)share;
+    const int64_t groups = (n + G - 1) / G;
+    for (int64_t g = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
+        const int64_t p = g * G + lane;
+        const bool mine = lane < G && p < n;
+        const int ci = mine ? a.cache_idx[p] : -1;
+        bool held = false;
+        int nh = 0;
+        int64_t checks = 0;
+        if (lane == 0) W.meet = 0;
         if (ci >= 0) {
             const double* ps = a.pose + 14 * p;
-            const V3 tpos[2] = {V3{ps[0], ps[1], ps[2]}, V3{ps[7], ps[8], ps[9]}};
-            const Q4 qn[2] = {qnormalize(Q4{ps[3], ps[4], ps[5], ps[6]}), qnormalize(Q4{ps[10], ps[11], ps[12], ps[13]})};
+            const double* e = a.cache_in + CACHE_W * (int64_t)ci;
             const int mesh[2] = {a.pmesh[2 * p], a.pmesh[2 * p + 1]};
             const double R[2] = {__longlong_as_double((long long)a.mesh_R_bits[mesh[0]]),
                                  __longlong_as_double((long long)a.mesh_R_bits[mesh[1]])};
             auto inf = [](V3 v) { return smax3(fabs(v.x), fabs(v.y), fabs(v.z)); };
-            const double pad = 1e-9 * (inf(tpos[0]) + inf(tpos[1]) + R[0] + R[1]);
-            const double* e = a.cache_in + CACHE_W * (int64_t)ci;
+            const double pad = 1e-9 * (inf(ld3(ps)) + inf(ld3(ps + 7)) + R[0] + R[1]);
             double mv = 0.0;
+#pragma unroll
             for (int s2 = 0; s2 < 2; ++s2) {
+                const double* q = ps + 7 * s2;
                 const double* o = e + 1 + 7 * s2;
+                const V3 x = ld3(q);
+                const Q4 qn = qnormalize(Q4{q[3], q[4], q[5], q[6]});
                 const Q4 q0 = qnormalize(Q4{o[3], o[4], o[5], o[6]});
-                mv += norm(tpos[s2] - V3{o[0], o[1], o[2]}) + 2.0 * R[s2] * qdist(qn[s2], q0);
+                mv += norm(x - V3{o[0], o[1], o[2]}) + 2.0 * R[s2] * qdist(qn, q0);
+                double* w = W.pose[lane] + 7 * s2;
+                w[0] = x.x, w[1] = x.y, w[2] = x.z;
+                w[3] = qn.w, w[4] = qn.x, w[5] = qn.y, w[6] = qn.z;
+                W.off[lane][s2] = a.tri_off[mesh[s2]];
             }
-            if (mv * (1.0 + 1e-9) + 8.0 * pad < e[0]) {
-                const int nh = (int)e[CACHE_NH];
-                const uint32_t* hin = a.cache_hin + CACHE_H * (int64_t)ci;
-                const int64_t off[2] = {a.tri_off[mesh[0]], a.tri_off[mesh[1]]};
-                bool meet = false;
-                for (int h = lane; h < nh; h += 32) {
-                    const uint32_t code = hin[h];
-                    const int tt[2] = {(int)(code >> 16), (int)(code & 0xffffu)};
-                    V3 W[2][3], nv[2];
-                    double d[2];
-                    bool ok = true;
-                    for (int s2 = 0; s2 < 2 && ok; ++s2) {
-                        const double* v = a.tris + 9 * (off[s2] + tt[s2]);
-                        for (int k = 0; k < 3; ++k) W[s2][k] = qrotate_n(qn[s2], ld3(v + 3 * k)) + tpos[s2];
-                        ok = plane_from_tri(W[s2][0], W[s2][1], W[s2][2], nv[s2], d[s2]) && !(norm2(nv[s2]) < 1e-30);
-                    }
-                    if (!ok) continue;  // a triangle without a plane: the full test drops it
-                    V3 lo[2], hi[2];
-                    for (int s2 = 0; s2 < 2; ++s2) {
-                        lo[s2] = V3{smin3(W[s2][0].x, W[s2][1].x, W[s2][2].x), smin3(W[s2][0].y, W[s2][1].y, W[s2][2].y),
-                                    smin3(W[s2][0].z, W[s2][1].z, W[s2][2].z)};
-                        hi[s2] = V3{smax3(W[s2][0].x, W[s2][1].x, W[s2][2].x), smax3(W[s2][0].y, W[s2][1].y, W[s2][2].y),
-                                    smax3(W[s2][0].z, W[s2][1].z, W[s2][2].z)};
-                    }
-                    const bool sep = hi[0].x < lo[1].x || lo[0].x > hi[1].x || hi[0].y < lo[1].y || lo[0].y > hi[1].y ||
-                                     hi[0].z < lo[1].z || lo[0].z > hi[1].z;
-                    V3 o0, o1;
-                    if (!sep && tri_tri(W[0], nv[0], d[0], W[1], nv[1], d[1], o0, o1)) meet = true;
-                }
-                if (!__any_sync(FULL, meet)) {
-                    flag = 1;
-                    const int nt1 = (int)(a.tri_off[mesh[1] + 1] - off[1]);
-                    if (lane == 0) {
-                        const int64_t checks = (int64_t)a.mesh_valid[mesh[0]] * nt1;
-                        a.pair_seg_off[p] = 0;
-                        a.pair_nseg[p] = 0;
-                        a.pair_checks[p] = checks;
-                        a.pair_status[p] = 0;
-                        atomicAdd(a.checks_total, (unsigned long long)checks);
-                        // what the rebuild writes for a pair without segments
-                        a.pair_stage_off[p] = 0;
-                        a.pair_pts_stage_off[p] = 0;
-                        a.pair_ncontact[p] = 0;
-                        a.pair_npts[p] = 0;
-                        a.pair_ncomp[p] = 0;
-                        a.pair_nloop[p] = 0;
-                    }
-                    // the entry carries over unchanged, marked as a skip
-                    if (lane < CACHE_W) a.cache_out[CACHE_W * p + lane] = lane == CACHE_SKIP ? 1.0 : e[lane];
-                    for (int h = lane; h < nh; h += 32) a.cache_hout[CACHE_H * p + h] = hin[h];
-                } else if (nh <= a.cap_side) {
-                    flag = 2;  // k_segments tests the near pairs alone
-                }
+            W.ci[lane] = ci;
+            held = mv * (1.0 + 1e-9) + 8.0 * pad < e[0];
+            if (held) {
+                nh = (int)e[CACHE_NH];
+                checks = (int64_t)a.mesh_valid[mesh[0]] * (int)(a.tri_off[mesh[1] + 1] - a.tri_off[mesh[1]]);
             }
         }
-        if (lane == 0) a.cache_skip[p] = flag;
+        // where each pair's near pairs begin among the warp's
+        int end = nh;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(FULL, end, d);
+            if (lane >= d) end += t;
+        }
+        const int beg = end - nh, total = __shfl_sync(FULL, end, 31);
+        __syncwarp();
+        for (int x0 = 0; x0 < total; x0 += 32) {
+            const int x = x0 + lane;
+            int own = 0;  // the last pair that begins at or before x
+#pragma unroll
+            for (int d = 16; d; d >>= 1) {
+                const int f = __shfl_sync(FULL, beg, own + d);
+                if (f <= x) own += d;
+            }
+            const int h = x - __shfl_sync(FULL, beg, own);
+            if (x < total && !(W.meet >> own & 1u)) {
+                const uint32_t code = a.cache_hin[CACHE_H * (int64_t)W.ci[own] + h];
+                // carried over (a pair that is tested after all gets its codes anew)
+                a.cache_hout[CACHE_H * (g * G + own) + h] = code;
+                const int tt[2] = {(int)(code >> 16), (int)(code & 0xffffu)};
+                V3 C[2][3], nv[2], lo[2], hi[2];
+                double d[2];
+#pragma unroll
+                for (int s2 = 0; s2 < 2; ++s2) {
+                    const double* w = W.pose[own] + 7 * s2;
+                    const Q4 q{w[3], w[4], w[5], w[6]};
+                    const double* v = a.tris + 9 * (W.off[own][s2] + tt[s2]);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) C[s2][k] = qrotate_n(q, ld3(v + 3 * k)) + ld3(w);
+                    lo[s2] = V3{smin3(C[s2][0].x, C[s2][1].x, C[s2][2].x), smin3(C[s2][0].y, C[s2][1].y, C[s2][2].y),
+                                smin3(C[s2][0].z, C[s2][1].z, C[s2][2].z)};
+                    hi[s2] = V3{smax3(C[s2][0].x, C[s2][1].x, C[s2][2].x), smax3(C[s2][0].y, C[s2][1].y, C[s2][2].y),
+                                smax3(C[s2][0].z, C[s2][1].z, C[s2][2].z)};
+                }
+                const bool sep = (hi[0].x < lo[1].x) | (lo[0].x > hi[1].x) | (hi[0].y < lo[1].y) | (lo[0].y > hi[1].y) |
+                                 (hi[0].z < lo[1].z) | (lo[0].z > hi[1].z);
+                if (!sep) {
+                    bool ok = true;  // a triangle without a plane: the full test drops it
+#pragma unroll
+                    for (int s2 = 0; s2 < 2; ++s2)
+                        ok &= plane_from_tri(C[s2][0], C[s2][1], C[s2][2], nv[s2], d[s2]) && !(norm2(nv[s2]) < 1e-30);
+                    V3 o0, o1;
+                    if (ok && tri_tri(C[0], nv[0], d[0], C[1], nv[1], d[1], o0, o1)) atomicOr(&W.meet, 1u << own);
+                }
+            }
+            __syncwarp();
+        }
+        const bool settled = held && !(W.meet >> lane & 1u);
+        if (settled) {
+            a.pair_seg_off[p] = 0;
+            a.pair_nseg[p] = 0;
+            a.pair_checks[p] = checks;
+            a.pair_status[p] = 0;
+            // what the rebuild writes for a pair without segments
+            a.pair_stage_off[p] = 0;
+            a.pair_pts_stage_off[p] = 0;
+            a.pair_ncontact[p] = 0;
+            a.pair_npts[p] = 0;
+            a.pair_ncomp[p] = 0;
+            a.pair_nloop[p] = 0;
+        } else {
+            checks = 0;
+        }
+        // 2: k_segments tests the near pairs alone
+        if (mine) a.cache_skip[p] = settled ? 1 : held && nh <= a.cap_side ? 2 : 0;
+#pragma unroll
+        for (int d = 16; d; d >>= 1) checks += __shfl_xor_sync(FULL, checks, d);
+        if (lane == 0 && checks) atomicAdd(a.checks_total, (unsigned long long)checks);
+        // the entries of settled pairs carry over unchanged, marked as a skip
+        const unsigned done = __ballot_sync(FULL, settled);
+        for (int i = lane; i < G * CACHE_W; i += 32) {
+            const int k = i / CACHE_W, w = i - k * CACHE_W;
+            if (done >> k & 1u)
+                a.cache_out[CACHE_W * (g * G + k) + w] = w == CACHE_SKIP ? 1.0 : a.cache_in[CACHE_W * (int64_t)W.ci[k] + w];
+        }
+        __syncwarp();
     }
 }
 

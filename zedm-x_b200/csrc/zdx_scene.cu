@@ -1701,7 +1701,7 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
             a.cache_tau = s.cfg.contact_cache_tau;
             a.cache_skip = as<int32_t>(G.cskip);
             a.order_count = reinterpret_cast<int*>(cnt + 8);
-            launch_cache_skip(a, std::max(1, ctx->num_sms) * 8, st);
+            launch_cache_skip(a, std::max(1, ctx->num_sms) * 3, st);
         }
         // a small scene's few pairs take the identity order that graph_alloc wrote
         if (s.np >= kCacheMinParticles) launch_cost_order(a, as<int32_t>(G.order), as<int>(G.buckets), st);
