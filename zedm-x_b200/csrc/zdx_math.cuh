@@ -253,6 +253,14 @@ ZDX_HD bool beyond_plane(V3 n, double d, V3 a, V3 b, V3 c, double m) {
                  s2 = n.x * c.x + n.y * c.y + n.z * c.z + d;
     return ((s0 > m) & (s1 > m) & (s2 > m)) | ((s0 < -m) & (s1 < -m) & (s2 < -m));
 }
+// How far triangle (a, b, c) lies on one side of the plane (n, d), negative when it reaches through: a lower bound
+// on its distance from any triangle in that plane.
+ZDX_HD double plane_gap(V3 n, double d, V3 a, V3 b, V3 c) {
+    const double s0 = n.x * a.x + n.y * a.y + n.z * a.z + d, s1 = n.x * b.x + n.y * b.y + n.z * b.z + d,
+                 s2 = n.x * c.x + n.y * c.y + n.z * c.z + d;
+    const double lo = smin3(s0, s1, s2), hi = smax3(s0, s1, s2);
+    return lo > -hi ? lo : -hi;
+}
 ZDX_HD bool tri_tri(const V3* A, V3 nA, double dA, const V3* B, V3 nB, double dB, V3& o0, V3& o1) {
     return tri_tri_src(A, nA, dA, B, nB, dB, o0, o1, nullptr, nullptr);
 }

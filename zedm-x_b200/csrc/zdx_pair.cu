@@ -261,6 +261,8 @@ __device__ __forceinline__ V3 slot_corner(const double* tri, int i, int k, int c
     return V3{tri[(3 * k) * cap + i], tri[(3 * k + 1) * cap + i], tri[(3 * k + 2) * cap + i]};
 }
 
+constexpr unsigned BOXES_APART = 0x80000000u;  // in a listed pair: CACHE lists it for its small gap alone
+
 // |q - q0| or |q + q0|, whichever is smaller (unit quaternions; a rotation and its negative are one)
 __device__ __forceinline__ double qdist(Q4 q, Q4 q0) {
     const double m = sqrt((q.w - q0.w) * (q.w - q0.w) + (q.x - q0.x) * (q.x - q0.x) + (q.y - q0.y) * (q.y - q0.y) +
@@ -678,9 +680,12 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
         // outgrow the list; then the window is halved and taken again.
         int r0 = 0, c0 = 0, rows = nA, cols = nB;
         bool boxes = nA <= K1<T>::BCAP && nB <= K1<T>::BCAP;  // the culls' boxes are all in shared memory
-        // CACHE: survivor pairs whose boxes are less than tau apart (those that met, and so every segment,
-        // included) become the entry's near pairs, tested again at every skip; the smallest box gap of the
-        // others (the largest separation over the axes, rounded down) bounds the entry's clearance
+        // CACHE: survivor pairs that neither their boxes nor one's plane hold tau apart (every segment's included)
+        // become the entry's near pairs, tested again at every skip; the smallest such gap of the others (box
+        // gaps: the largest separation over the axes, rounded down) bounds the entry's clearance.  A gap from a
+        // plane is one between the triangles, so what the two move by may come off it as off a box gap.  With box
+        // gaps alone a touching pair had more near pairs than an entry holds and was tested whole at each step:
+        // of the pour's 87,000 pairs 83,500 instead of 75,500 now hold an entry, 1.13 -> 0.50 ms a step.
         float gmin = __int_as_float(0x7f800000);
         const float near_gap = CACHE ? __double2float_ru(tau) : 0.f;
         for (;;) {
@@ -809,13 +814,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                                                                   fmaxf(__fsub_rd(b4.y, q.x), __fsub_rd(p.y, b2.x))),
                                                             fmaxf(__fsub_rd(b4.z, q.y), __fsub_rd(p.z, b2.y)));
                                     if (live & !(gap >= near_gap)) {
-                                        const int ta = SA.id[a0 + i], tb = SB.id[b0 + ob];
-                                        const int h = atomicAdd(&sh_nh, 1);
-                                        if (ta < 65536 && tb < 65536 && h < CACHE_H)
-                                            a.cache_hout[CACHE_H * (int64_t)pair + h] = (uint32_t)ta << 16 | (uint32_t)tb;
-                                        else
-                                            sh_cbad = 1;
-                                        if (!(gap > 0.f)) found(a0 + i, b0 + ob);
+                                        found(a0 + i, gap > 0.f ? (b0 + ob) | BOXES_APART : b0 + ob);
                                     } else if (live) {
                                         gmin = fminf(gmin, gap);
                                     }
@@ -833,16 +832,39 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                 if (rows > 1) rows = (rows + 1) >> 1;
                 else cols = (cols + 1) >> 1;
                 __syncthreads();
-                if (tid == 0) {
-                    sh_nq = 0;
-                    if constexpr (CACHE) sh_cbad = 1;  // its near pairs are listed already
-                }
+                if (tid == 0) sh_nq = 0;
                 __syncthreads();
                 continue;
             }
             // ---- the listed pairs: the reference's box test, then the planes
             for (int q = tid; q < nq; q += T) {
-                const uint2 e = S.list[0][q];
+                uint2 e = S.list[0][q];
+                if constexpr (CACHE) {
+                    const bool apart = e.y & BOXES_APART;
+                    e.y &= ~BOXES_APART;
+                    // how far one triangle lies beyond the other's plane, less what point_in_tri adds to either
+                    const int ta = SA.id[e.x], tb = SB.id[e.y];
+                    auto gap = [&](const K1Side& P, int i, const K1Side& U, int j) {
+                        return plane_gap(V3{P.pl[i], P.pl[cap + i], P.pl[2 * cap + i]}, P.pl[3 * cap + i],
+                                         slot_corner(U.tri, j, 0, cap), slot_corner(U.tri, j, 1, cap),
+                                         slot_corner(U.tri, j, 2, cap));
+                    };
+                    const double infl = fmax(a.tri_infl[off[0] + ta], a.tri_infl[off[1] + tb]);
+                    const double clear = fmax(gap(SB, e.y, SA, e.x), gap(SA, e.x, SB, e.y)) - infl - 8.0 * pad;
+                    if (clear >= tau) {
+                        gmin = fminf(gmin, __double2float_rd(clear));
+                    } else {
+                        const int h = atomicAdd(&sh_nh, 1);
+                        if (ta < 65536 && tb < 65536 && h < CACHE_H)
+                            a.cache_hout[CACHE_H * (int64_t)pair + h] = (uint32_t)ta << 16 | (uint32_t)tb;
+                        else
+                            sh_cbad = 1;
+                    }
+                    // beyond the plane: no segment, whatever the boxes do
+                    if (apart || clear > 0.0 || !meets(e.x, e.y)) continue;
+                    S.list[1][atomicAdd(&sh_nt, 1)] = e;
+                    continue;
+                }
                 if (!meets(e.x, e.y)) continue;
                 if (a.tri_infl) {
                     const double more = 8.0 * pad;
@@ -1081,7 +1103,9 @@ constexpr int CSKIP_PAIRS = 16;
 // motion, then over all their near pairs, one behind the other, until one of a pair's meets.  Bound: FP64
 // instructions (issue 0.49, a third of the FP64 pipe's cycles) and the near pairs' corners, which L1 and L2 hold.
 // With a warp per pair the motion (four normalised quaternions in a row) ran on every lane alike and a pair's last
-// near pairs left lanes idle: 87,000 pairs of the pour, 0.40 ms.  Shared out: 0.228 ms.
+// near pairs left lanes idle: 87,000 pairs of the pour, 0.40 ms.  Shared out: 0.228 ms with 32 a warp, 0.17 with the
+// near pairs that planes leave (k_segments) and 16 or 8 a warp, 0.21 with 4 (a warp's tail then decides).  The
+// planes tested here before tri_tri: no gain.
 struct CacheSkipWarp {
     double pose[CSKIP_PAIRS][15];  // positions and unit quaternions of A and B (one word of padding: banks)
     int64_t off[CSKIP_PAIRS][2];   // first triangles
