@@ -183,7 +183,7 @@ PROFILED = {
     "k_rebuild": {"warp_inst_per_pair": 147357.0, "dram_bytes_per_pair": 17377.0},
 }
 KERNEL_SOURCES = ("zdx_pair.cu", "zdx_pair.cuh", "zdx_math.cuh", "zdx_npmath.cuh", "zdx_pyset.cuh",
-                  "zdx_sortrep.cuh", "zdx_radix.cuh")
+                  "zdx_sortrep.cuh", "zdx_radix.cuh", "zdx_team.cu", "zdx_team.cuh")
 
 
 def kernel_sources_sha256():
@@ -511,11 +511,17 @@ def main():
                          reb_ms, step_ms, base_cfg, extras))
         return
     # parity of this step's output with the reference's own code on the CPU baseline's sample
-    rate, n_cpu, dt_cpu, sel, rec = cpu_reference_rate(lib, pm, pp, 1, args.cpu_seconds, record=True)
-    extras["cpu_baseline"] = {"value": rate, "unit": UNIT, "cores": 1, "kind": "reference",
-                              "sample": f"{n_cpu} random pairs of the workload through oracle/_ref, {dt_cpu:.1f} s"}
-    extras["parity"] = parity_check(sel, rec, res["stats"], res["contact_off"], res["geom"])
-    log(f"parity: {extras['parity']['pairs']} pairs, {extras['parity']['mismatches']} mismatches")
+    from oracle import LIB_REF
+
+    if os.path.exists(LIB_REF):
+        rate, n_cpu, dt_cpu, sel, rec = cpu_reference_rate(lib, pm, pp, 1, args.cpu_seconds, record=True)
+        extras["cpu_baseline"] = {"value": rate, "unit": UNIT, "cores": 1, "kind": "reference",
+                                  "sample": f"{n_cpu} random pairs of the workload through oracle/_ref, {dt_cpu:.1f} s"}
+        extras["parity"] = parity_check(sel, rec, res["stats"], res["contact_off"], res["geom"])
+        log(f"parity: {extras['parity']['pairs']} pairs, {extras['parity']['mismatches']} mismatches")
+    else:
+        extras["cpu_baseline"] = extras["parity"] = {
+            "unavailable": "oracle/_ref is not built (make -C oracle ref needs the reference's sources)"}
     extras.update(sweep_comparisons(args, ctx, dev, meshes, pairs, out, res, flush, step_ms))
     extras["strong_shards"] = shard_balance(args, ctx, dev, meshes, pairs, flush, statistics.mean(step_ms))
     log("strong shards: " + ", ".join(f"{k} {v['balance_mean_over_max']:.3f}" for k, v in extras["strong_shards"].items()

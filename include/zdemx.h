@@ -166,8 +166,8 @@ int zdx_get_stream(const zdx_ctx* ctx, void** stream);
  * that cannot be read or parsed is ignored).  A scene's graph step keeps the values in force when the
  * scene was loaded. */
 typedef struct zdx_tuning {
-    int32_t tri_ctas_per_sm;    /* triangle-stage CTAs per SM: 1 or 2 (default 2)                     */
-    int32_t rebuild_warps;      /* warps per rebuild block, 1..4 (default 4)                          */
+    int32_t tri_ctas_per_sm;    /* triangle-stage CTAs per SM: 1, or 2 (default) for as many as fit    */
+    int32_t rebuild_warps;      /* warps per rebuild block, 1..4 (default 4), where a warp takes a pair */
     int64_t flat_max;           /* survivor pairs nA' x nB' up to which the flat box test runs rather
                                    than the hierarchical one (default 262144)                        */
     int64_t split_tests;        /* a batch with fewer pairs than triangle-stage CTAs splits each pair
@@ -176,13 +176,14 @@ typedef struct zdx_tuning {
                                    (default).  zdx_pair_contacts only                                 */
     int32_t rebuild_arena;      /* rebuild form of zdx_pair_contacts in zdem mode (without adjoint tape,
                                    loop points or component stats), same results in every form: 0
-                                   (default) one warp per pair with its arrays in a global-memory slot;
+                                   (default) blocks taking packs of pairs in shared memory, then one
+                                   warp per pair with its arrays in a global-memory slot for the pairs
+                                   no block holds;
                                    1 pairs of at least arena_min_seg segments in arenas (one warp per
                                    pair: the neighbour relation from a sorted sweep, a lock-free
                                    union-find for the snap), on a second stream at the same time as
-                                   form 0 on the smaller pairs; 2 every pair in an arena (fastest when
-                                   most pairs have hundreds of segments); 3 an arena too small for any
-                                   pair, so that every pair with segments falls back to form 0 (a test
+                                   the warps of form 0 on the smaller pairs; 2 every pair in an arena; 3 an arena too small for any
+                                   pair, so that every pair with segments falls back to form 0's warps (a test
                                    of that path)                                                     */
     int32_t arena_warps;        /* warps per SM given arenas, 1..32 (default 8)                      */
     int32_t arena_min_seg;      /* form 1: pairs of fewer segments take form 0 (default 192)        */

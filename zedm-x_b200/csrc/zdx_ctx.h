@@ -25,7 +25,7 @@ struct Scene;  // DEM scene (zdx_scene.cu)
 
 // Launch parameters of the pair kernels (zdx_set_tuning; defaults measured on the pair sweep).
 struct Tuning {
-    int tri_ctas_per_sm = 2;     // triangle-stage CTAs per SM (shared memory allows 1 or 2)
+    int tri_ctas_per_sm = 2;     // triangle-stage CTAs per SM: 1, or 2 for as many as fit (triangle_ctas)
     int64_t flat_max = 262144;   // survivor pairs up to which the flat box test beats the hierarchical one
     int rebuild_warps = 4;       // warps per rebuild block
     int64_t split_tests = 0;     // split a pair's triangle stage into chunks of about this many survivor

@@ -3,15 +3,18 @@
 // packs of pairs, and the pairs no class holds are left to the warp-per-pair kernel of zdx_pair.cu.
 //
 // What bounds it: latency (chains of shared-memory loads on a warp in the searches and walks, FP64 divides, about
-// 40 barriers a pack), an issue rate of a fifth to a quarter.  The warp-per-pair kernel waited on L1 and L2 for
+// 40 barriers a pack: 6 of 14 stall cycles an issue), a third of the issue slots used.  The warp-per-pair kernel waited on L1 and L2 for
 // the same chains and spent 1,490 warp instructions a segment on scans that this form replaces by lists (about
 // 300).  A pack rather than a pair a block: small pairs a warp each had 12 of 32 lanes live and half their stalls
 // on instruction fetch, as every warp of an SM was somewhere else in the code.  Three 256-thread blocks an SM
 // (80 registers): 128-thread blocks (six an SM, packs of 190 segments) 16.7 ms, two blocks an SM with packs of
 // 560 segments 17.0 (256 threads) and 16.9 ms (512) against 16.1 on the pair sweep.
-// Rebuild stage on a B200, warp-per-pair kernel against this: 65,536-pair sweep (103 segments a pair) 27.2 -> 13.0
+// With the walks, claims and searches of zdx_team.cuh as they are now the first class with 128-thread blocks takes
+// 14.4 ms and with 192-thread ones 13.6 against 12.7; the code with its loops rolled up (157 instead of 177 KB) 13.8
+// against 13.0.
+// Rebuild stage on a B200, warp-per-pair kernel against this: 65,536-pair sweep (103 segments a pair) 27.2 -> 11.0
 // ms, 1,500 pairs of 5,120-triangle meshes (400 segments) 6.7 -> 1.8, 16,384 pairs of 320-triangle ones (25)
-// 1.79 -> 0.54, 64 mixed pairs 3.85 -> 0.50, one pair of 320-triangle meshes 0.14 -> 0.06.
+// 1.79 -> 0.45, 64 mixed pairs 3.85 -> 0.49, one pair of 320-triangle meshes 0.14 -> 0.06.
 //
 // Compiled with --fmad=false: see zdx_math.cuh.
 #include "zdx_team.cuh"
