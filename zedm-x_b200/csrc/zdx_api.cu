@@ -117,10 +117,9 @@ extern "C" int zdx_destroy(zdx_ctx* ctx) {
     ctx->scene_release();
     for (auto& e : ctx->ev) cudaEventDestroy(e);
     cudaStreamDestroy(ctx->stream);
-    if (ctx->stream2) {
-        for (auto& e : ctx->ev2) cudaEventDestroy(e);
-        cudaStreamDestroy(ctx->stream2);
-    }
+    for (auto& e : ctx->ev2)
+        if (e) cudaEventDestroy(e);
+    if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
     delete ctx;
     return ZDX_OK;
 }
@@ -140,6 +139,15 @@ int tuning_check(const zdx_tuning* t) {
     if (t->flat_max < 0 || t->split_tests < 0) return ZDX_ERR_INVALID;
     if (t->rebuild_arena < 0 || t->rebuild_arena > 3 || t->arena_warps < 1 || t->arena_warps > 32) return ZDX_ERR_INVALID;
     if (t->arena_min_seg < 0 || t->arena_pad != 0) return ZDX_ERR_INVALID;
+    return ZDX_OK;
+}
+
+// The rebuild's second stream, created on first use.
+int second_stream(zdx_ctx* ctx) {
+    if (ctx->stream2) return ZDX_OK;
+    for (auto& e : ctx->ev2)
+        if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
     return ZDX_OK;
 }
 
@@ -167,10 +175,7 @@ int rebuild_by_arenas(zdx_ctx* ctx, PairArgs a, int64_t NP, int nmax, size_t bud
     CK(ctx->ar_gslots.ensure((size_t)plan.arena_bytes * (size_t)slots));
     plan.gslots = static_cast<char*>(ctx->ar_gslots.p);
     plan.grid = (int)(slots / 4);
-    if (!ctx->stream2) {
-        CK(cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking));
-        for (auto& e : ctx->ev2) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
+    if (int rc = second_stream(ctx)) return rc;
     // meanwhile the small pairs on the warp-per-pair kernel, with slots sized for them; afterwards the
     // pairs no arena held, with slots for the call's largest pair (one buffer, sized before either runs)
     struct WarpLaunch {
@@ -647,7 +652,11 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
             int st_code = rebuild_by_arenas(ctx, a, NP, nmax, budget, st);
             if (st_code != ZDX_OK) return st_code;
         } else if (teams) {
-            ctx->launches += launch_rebuild_teams(a, plan, ctx->num_sms, NP, nmax, st);
+            const bool fork = team_classes_of(nmax) > 1;
+            if (fork)
+                if (int rc = second_stream(ctx)) return rc;
+            const TeamSide side{ctx->stream2, {ctx->ev2[0], ctx->ev2[1]}};
+            ctx->launches += launch_rebuild_teams(a, plan, ctx->num_sms, NP, nmax, st, fork ? &side : nullptr);
         } else {
             int st_code = warp_form(a.order, NP);
             if (st_code != ZDX_OK) return st_code;

@@ -42,7 +42,7 @@ struct zdx_ctx {
     int num_sms = 148;
     int cc_major = 0, cc_minor = 0;
     cudaStream_t stream = nullptr;
-    cudaStream_t stream2 = nullptr;  // the arena rebuild's stream (created on first use)
+    cudaStream_t stream2 = nullptr;  // the rebuild's second stream (created on first use)
     cudaEvent_t ev2[2] = {};
     cudaEvent_t ev[8] = {};
     std::string last_error;

@@ -180,7 +180,14 @@ struct TeamPlan {
     int* counts;     // TEAM_COUNTS ints, zero before the launch: list lengths, from 8 on the classes' queues
 };
 constexpr int TEAM_COUNTS = 16;
-int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s);
+// With `side` (for a call of several classes), on a second stream too (forked from s and joined to it by the two events).
+struct TeamSide {
+    cudaStream_t stream;
+    cudaEvent_t ev[2];
+};
+int team_classes_of(int nmax);  // classes that pairs of up to nmax segments take
+int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s,
+                         const TeamSide* side = nullptr);
 // Bytes of one triangle-stage slot.
 size_t tritest_slot_bytes(int cap_side, int cap_seg);
 // Threads of a triangle-stage CTA for a batch (PairArgs::k1_threads), and the CTAs an SM runs for the tuning value

@@ -12,9 +12,9 @@
 // With the walks, claims and searches of zdx_team.cuh as they are now the first class with 128-thread blocks takes
 // 14.4 ms and with 192-thread ones 13.6 against 12.7; the code with its loops rolled up (157 instead of 177 KB) 13.8
 // against 13.0.
-// Rebuild stage on a B200, warp-per-pair kernel against this: 65,536-pair sweep (103 segments a pair) 27.2 -> 11.0
-// ms, 1,500 pairs of 5,120-triangle meshes (400 segments) 6.7 -> 1.8, 16,384 pairs of 320-triangle ones (25)
-// 1.79 -> 0.45, 64 mixed pairs 3.85 -> 0.49, one pair of 320-triangle meshes 0.14 -> 0.06.
+// Rebuild stage on a B200, warp-per-pair kernel against this: 65,536-pair sweep (103 segments a pair) 27.2 -> 10.1
+// ms, 1,500 pairs of 5,120-triangle meshes (400 segments) 6.7 -> 1.6, 16,384 pairs of 320-triangle ones (25)
+// 1.79 -> 0.45, 64 mixed pairs 3.85 -> 0.31, one pair of 320-triangle meshes 0.14 -> 0.06.
 //
 // Compiled with --fmad=false: see zdx_math.cuh.
 #include "zdx_team.cuh"
@@ -151,23 +151,40 @@ void launch_class(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, 
     k<<<(unsigned)(most < grid ? most : grid), c.threads, c.bytes, s>>>(a, pl, C, c.pack_seg, c.bytes);
 }
 
+// The classes share nothing but counters, and each ends with the chains of its last pairs on an idle chip: with a
+// second stream the classes of large pairs run beside the first.  Rebuild stage with one stream and with two: 65,536-pair
+// sweep 11.1 and 10.1 ms, 1,500 pairs of 5,120-triangle meshes 1.82 and 1.59, 64 mixed pairs 0.49 and 0.31.  A call
+// of one class keeps to one stream (a second one in the context cost the single-pair call 0.06 of 0.45 ms).
 template <bool NPX>
-int launch_classes(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s) {
+int launch_classes(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s,
+                   const TeamSide* side) {
     // blocks an SM holds: 227 KB over the class's memory, 5 KB of its own and the system's
+    const int n = team_classes_of(nmax);
+    const cudaStream_t s2 = side ? side->stream : s;
+    if (side) {
+        cudaEventRecord(side->ev[0], s);
+        cudaStreamWaitEvent(s2, side->ev[0], 0);
+    }
+    if (n > 2) launch_class<2, 1, NPX>(a, pl, sms, most, s2);
+    if (n > 1) launch_class<1, 2, NPX>(a, pl, sms, most, s2);
     launch_class<0, 3, NPX>(a, pl, sms, most, s);
-    if (nmax <= team_class(0).max_seg) return 1;
-    launch_class<1, 2, NPX>(a, pl, sms, most, s);
-    if (nmax <= team_class(1).max_seg) return 2;
-    launch_class<2, 1, NPX>(a, pl, sms, most, s);
-    return 3;
+    if (side) {
+        cudaEventRecord(side->ev[1], s2);
+        cudaStreamWaitEvent(s, side->ev[1], 0);
+    }
+    return n;
 }
 
 }  // namespace
 
-int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s) {
+int team_classes_of(int nmax) { return nmax <= team_class(0).max_seg ? 1 : nmax <= team_class(1).max_seg ? 2 : 3; }
+
+int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s,
+                         const TeamSide* side) {
     if (most <= 0) return 0;
     k_team_classes<<<(unsigned)((most + 255) / 256), 256, 0, s>>>(a, pl);
-    return 1 + (a.mode == 2 ? launch_classes<true>(a, pl, sms, most, nmax, s) : launch_classes<false>(a, pl, sms, most, nmax, s));
+    return 1 + (a.mode == 2 ? launch_classes<true>(a, pl, sms, most, nmax, s, side)
+                            : launch_classes<false>(a, pl, sms, most, nmax, s, side));
 }
 
 }  // namespace zdx
