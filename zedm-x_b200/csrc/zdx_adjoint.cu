@@ -83,7 +83,7 @@ __device__ __forceinline__ V3 scatter_corner(const AdjointArgs& a, const Body& b
     return cross(w - b.x, g);
 }
 
-// One warp per contact.  Bound: instructions in FP64 (some 1750 per endpoint, a third of them divisions) at the
+// One warp per contact.  Bound: instructions in FP64 (some 1,750 per endpoint) at the
 // lanes they fill.  Lanes over vertices, each walking its endpoints, filled 8.7 of 32 (the walks end apart and
 // do not meet again); lanes over the endpoints of 32 vertices, the owner found among the lanes' first
 // endpoints, take 49 instead of 164 million warp instructions: 16,384 pairs of 320-triangle meshes (24
