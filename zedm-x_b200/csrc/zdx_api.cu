@@ -402,7 +402,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     a.mesh_infl_bits = per_stage ? nullptr : as<unsigned long long>(ctx->mesh_infl);
     a.per_stage = per_stage ? 1 : 0;
     a.tri_sph = as<double4>(ctx->tri_sph);
-    a.tri_infl = per_stage ? nullptr : reinterpret_cast<float*>(a.tri_sph + std::max<int64_t>(total_tris, 1));
+    a.tri_reach = per_stage ? nullptr : reinterpret_cast<float*>(a.tri_sph + std::max<int64_t>(total_tris, 1));
     a.mesh_R_bits = as<unsigned long long>(ctx->mesh_R);
     a.mesh_valid = as<int>(ctx->mesh_valid);
     launch_mesh_prep(a, total_tris, st);

@@ -244,17 +244,37 @@ ZDX_HD double tri_inflation(V3 p0, V3 p1, V3 p2) {
     if (!(infl < 1e300)) infl = 1e300;
     return infl * (1.0 + 1e-6);
 }
+// How far outside a triangle, along its computed plane, the exact tests may accept a point, for the plane tests below:
+// tri_inflation with the rounding of point_in_tri's products added to its 1e-10.  The cross product is off by some eps l^2
+// (l: the longest edge), which tilts the normal of a thin triangle by eps l^2 over twice its area; where that is no small
+// angle its plane says nothing about the triangle: infinite.  (64 eps covers the products, the differences and a
+// rotation's roundings.)
+ZDX_HD double tri_reach(V3 p0, V3 p1, V3 p2) {
+    const V3 e0 = p1 - p0, e1 = p2 - p1, e2 = p0 - p2;
+    const double l = smax3(norm(e0), norm(e1), norm(e2));
+    const double round = 64.0 * 2.220446049250313e-16 * l * l;
+    if (!(round / norm(cross(e0, e2)) < 0.01)) return __builtin_huge_val();
+    return 1.001 * tri_inflation(p0, p1, p2) * (1.0 + 1e10 * round);
+}
+// How far a triangle's own corners can stand off its computed plane, from its reach and the radius R of its mesh:
+// by the tilt times l, 64 eps l^3 / (2 area), which is at most 7.2e-5 l^2 of the reach (2e-10 l^2 / (2 area l) and
+// more), and l is at most 2 R.  A sliver of length 0.9 and width 1e-9 stands off by 1.5e-7.
+ZDX_HD double plane_off(double reach, double R) { return 3e-4 * R * R * reach; }
+// Whether the reaches hold where the bodies are (pad: 1e-9 of the coordinates' size): rounding of the placed corners
+// must not change a sliver's width (2e-10 / reach or more) by more than a hundredth.
+ZDX_HD bool reaches_hold(double reachA, double reachB, double pad) { return smax(reachA, reachB) * pad < 4e-6; }
 // Whether the plane (n, d) of one triangle rules out a segment with triangle (a, b, c): its corners all lie on one
 // side, further than m.  Then no edge of it meets the plane (t is beyond [0, 1] by at least m over the edge, and m
-// covers 1e-10 edges), and no point of the plane lies in it, not even by point_in_tri's tolerance, which moves its
-// edges out by less than m.
+// covers 1e-10 edges).  The plane's owner has edges too, which are cut with the computed plane of (a, b, c): what is
+// accepted there lies on the owner, so within the owner's plane_off of (n, d), and within the reach and the plane_off of
+// (a, b, c).  m has to cover all three: with the reach alone segments of slivers were lost.
 ZDX_HD bool beyond_plane(V3 n, double d, V3 a, V3 b, V3 c, double m) {
     const double s0 = n.x * a.x + n.y * a.y + n.z * a.z + d, s1 = n.x * b.x + n.y * b.y + n.z * b.z + d,
                  s2 = n.x * c.x + n.y * c.y + n.z * c.z + d;
     return ((s0 > m) & (s1 > m) & (s2 > m)) | ((s0 < -m) & (s1 < -m) & (s2 < -m));
 }
-// How far triangle (a, b, c) lies on one side of the plane (n, d), negative when it reaches through: a lower bound
-// on its distance from any triangle in that plane.
+// How far triangle (a, b, c) lies on one side of the plane (n, d), negative when it reaches through: less the owner's
+// plane_off, a lower bound on its distance from the triangle that the plane was computed from.
 ZDX_HD double plane_gap(V3 n, double d, V3 a, V3 b, V3 c) {
     const double s0 = n.x * a.x + n.y * a.y + n.z * a.z + d, s1 = n.x * b.x + n.y * b.y + n.z * b.z + d,
                  s2 = n.x * c.x + n.y * c.y + n.z * c.z + d;

@@ -156,7 +156,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     a.mean_edge = ms->mean_edge;
     a.bbox_diag = ms->bbox_diag;
     a.tri_sph = cv.take<double4>(ZDX_NOALLOC_MAX_TRIS);
-    a.tri_infl = cv.take<float>(ZDX_NOALLOC_MAX_TRIS);
+    a.tri_reach = cv.take<float>(ZDX_NOALLOC_MAX_TRIS);
     a.mesh_R_bits = cv.take<unsigned long long>(ZDX_NOALLOC_MAX_MESHES);
     a.mesh_valid = cv.take<int>(ZDX_NOALLOC_MAX_MESHES);
     a.n_pairs = NP;

@@ -82,11 +82,10 @@ __global__ void k_mesh_prep(PairArgs a, int64_t total) {
         a.tri_sph[t] = make_double4(c.x, c.y, c.z, r);
         Rb = (unsigned long long)__double_as_longlong((norm(c) + r) * (1.0 + 1e-12));
         valid = !(norm(cross(p1 - p0, p2 - p0)) < 1e-30) ? 1 : 0;
-        if (a.tri_infl && !valid) a.tri_infl[t] = __int_as_float(0x7f800000);
+        if (a.tri_reach && !valid) a.tri_reach[t] = __int_as_float(0x7f800000);
         if (a.mesh_infl_bits && valid) {
-            const double infl = tri_inflation(p0, p1, p2);
-            ib = (unsigned long long)__double_as_longlong(infl);
-            if (a.tri_infl) a.tri_infl[t] = __double2float_ru(infl);
+            ib = (unsigned long long)__double_as_longlong(tri_inflation(p0, p1, p2));
+            if (a.tri_reach) a.tri_reach[t] = __double2float_ru(zdx::tri_reach(p0, p1, p2));
         }
     }
     // A mesh's triangles are consecutive, so they are runs of lanes: reduce each run (max, sum, max of
@@ -842,15 +841,17 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                 if constexpr (CACHE) {
                     const bool apart = e.y & BOXES_APART;
                     e.y &= ~BOXES_APART;
-                    // how far one triangle lies beyond the other's plane, less what point_in_tri adds to either
+                    // how far one triangle lies beyond the other's plane, less what either takes for itself
                     const int ta = SA.id[e.x], tb = SB.id[e.y];
                     auto gap = [&](const K1Side& P, int i, const K1Side& U, int j) {
                         return plane_gap(V3{P.pl[i], P.pl[cap + i], P.pl[2 * cap + i]}, P.pl[3 * cap + i],
                                          slot_corner(U.tri, j, 0, cap), slot_corner(U.tri, j, 1, cap),
                                          slot_corner(U.tri, j, 2, cap));
                     };
-                    const double infl = fmax(a.tri_infl[off[0] + ta], a.tri_infl[off[1] + tb]);
-                    const double clear = fmax(gap(SB, e.y, SA, e.x), gap(SA, e.x, SB, e.y)) - infl - 8.0 * pad;
+                    const double rA = a.tri_reach[off[0] + ta], rB = a.tri_reach[off[1] + tb];
+                    const double oA = plane_off(rA, R[0]), oB = plane_off(rB, R[1]);
+                    double clear = fmax(gap(SB, e.y, SA, e.x) - oB, gap(SA, e.x, SB, e.y) - oA) - fmax(rA + oA, rB + oB) - 8.0 * pad;
+                    if (!reaches_hold(rA, rB, pad)) clear = -1.0;
                     if (clear >= tau) {
                         gmin = fminf(gmin, __double2float_rd(clear));
                     } else {
@@ -866,16 +867,16 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                     continue;
                 }
                 if (!meets(e.x, e.y)) continue;
-                if (a.tri_infl) {
-                    const double more = 8.0 * pad;
+                if (a.tri_reach) {
+                    const double rA = a.tri_reach[off[0] + SA.id[e.x]], rB = a.tri_reach[off[1] + SB.id[e.y]];
+                    const double more = plane_off(rA, R[0]) + plane_off(rB, R[1]) + 8.0 * pad;
                     auto beyond = [&](const K1Side& P, int i, const K1Side& U, int j, double m) {
                         return beyond_plane(V3{P.pl[i], P.pl[cap + i], P.pl[2 * cap + i]}, P.pl[3 * cap + i],
                                             slot_corner(U.tri, j, 0, cap), slot_corner(U.tri, j, 1, cap),
                                             slot_corner(U.tri, j, 2, cap), m);
                     };
-                    const bool far0 = beyond(SB, e.y, SA, e.x, a.tri_infl[off[0] + SA.id[e.x]] + more);
-                    const bool far1 = beyond(SA, e.x, SB, e.y, a.tri_infl[off[1] + SB.id[e.y]] + more);
-                    if (far0 | far1) continue;
+                    const bool far0 = beyond(SB, e.y, SA, e.x, rA + more), far1 = beyond(SA, e.x, SB, e.y, rB + more);
+                    if ((far0 | far1) & reaches_hold(rA, rB, pad)) continue;
                 }
                 S.list[1][atomicAdd(&sh_nt, 1)] = e;
             }

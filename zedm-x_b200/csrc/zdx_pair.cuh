@@ -33,9 +33,9 @@ struct PairArgs {
     const double* bbox_diag;
     // per-triangle bounding spheres (cx, cy, cz, r) in the mesh frame and per-mesh bounds (k_mesh_prep)
     double4* tri_sph;
-    // per triangle, how far outside it point_in_tri's tolerance can accept a point (rounded up; k_mesh_prep);
-    // null with mesh_infl_bits
-    float* tri_infl;
+    // per triangle, how far outside it a point may be accepted (zdx::tri_reach, rounded up; k_mesh_prep); null with
+    // mesh_infl_bits
+    float* tri_reach;
     unsigned long long* mesh_R_bits;  // max over triangles of |c| + r, as the bits of a positive double
     int* mesh_valid;                  // triangles with a plane (|e1 x e2| >= 1e-30) per mesh
     // per mesh, how far outside a triangle point_in_tri's tolerance can accept a point (bits of a

@@ -1577,7 +1577,7 @@ static int graph_alloc(zdx_ctx* ctx, Scene& s) {
         m.tris = as<double>(s.d_mtris);
         m.tri_off = as<int64_t>(s.d_moff);
         m.tri_sph = as<double4>(G.tri_sph);
-        m.tri_infl = reinterpret_cast<float*>(m.tri_sph + std::max<int64_t>(total_tris, 1));
+        m.tri_reach = reinterpret_cast<float*>(m.tri_sph + std::max<int64_t>(total_tris, 1));
         m.mesh_R_bits = as<unsigned long long>(G.mesh_R);
         m.mesh_valid = as<int>(G.mesh_valid);
         m.mesh_infl_bits = as<unsigned long long>(G.mesh_infl);
@@ -1649,7 +1649,7 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         a.mean_edge = as<double>(s.d_mme);
         a.bbox_diag = as<double>(s.d_mbd);
         a.tri_sph = as<double4>(G.tri_sph);
-        a.tri_infl = reinterpret_cast<float*>(a.tri_sph + std::max<int64_t>(s.mesh_off.back(), 1));
+        a.tri_reach = reinterpret_cast<float*>(a.tri_sph + std::max<int64_t>(s.mesh_off.back(), 1));
         a.mesh_R_bits = as<unsigned long long>(G.mesh_R);
         a.mesh_valid = as<int>(G.mesh_valid);
         a.n_pairs = G.pcap;
