@@ -812,7 +812,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                                     const float gap = fmaxf(fmaxf(fmaxf(__fsub_rd(b4.x, p.w), __fsub_rd(p.x, b4.w)),
                                                                   fmaxf(__fsub_rd(b4.y, q.x), __fsub_rd(p.y, b2.x))),
                                                             fmaxf(__fsub_rd(b4.z, q.y), __fsub_rd(p.z, b2.y)));
-                                    if (live & !(gap >= near_gap)) {
+                                    if (live & !((gap >= near_gap) & (gap > 0.f))) {  // boxes that touch meet
                                         found(a0 + i, gap > 0.f ? (b0 + ob) | BOXES_APART : b0 + ob);
                                     } else if (live) {
                                         gmin = fminf(gmin, gap);
@@ -852,7 +852,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                     const double oA = plane_off(rA, R[0]), oB = plane_off(rB, R[1]);
                     double clear = fmax(gap(SB, e.y, SA, e.x) - oB, gap(SA, e.x, SB, e.y) - oA) - fmax(rA + oA, rB + oB) - 8.0 * pad;
                     if (!reaches_hold(rA, rB, pad)) clear = -1.0;
-                    if (clear >= tau) {
+                    if (clear >= tau && clear > 0.0) {
                         gmin = fminf(gmin, __double2float_rd(clear));
                     } else {
                         const int h = atomicAdd(&sh_nh, 1);

@@ -1698,7 +1698,8 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
             a.cache_out = as<double>(G.cout);
             a.cache_hin = as<uint32_t>(G.chit);
             a.cache_hout = as<uint32_t>(G.chout);
-            a.cache_tau = s.cfg.contact_cache_tau;
+            // none, and no number, is no margin: the culls must not drop what they would without it
+            a.cache_tau = s.cfg.contact_cache_tau > 0.0 ? s.cfg.contact_cache_tau : 0.0;
             a.cache_skip = as<int32_t>(G.cskip);
             a.order_count = reinterpret_cast<int*>(cnt + 8);
             launch_cache_skip(a, std::max(1, ctx->num_sms) * 3, st);
