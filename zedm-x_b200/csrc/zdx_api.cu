@@ -521,8 +521,12 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
         k1_grid = (int)std::min<int64_t>((int64_t)ni, ctas);
         CK(cudaStreamSynchronize(st));  // the host vectors go out of scope
     }
-    a.k1_slot_bytes = tritest_slot_bytes(a.cap_side, a.cap_seg);
-    CK(ctx->k1_slots.ensure(a.k1_slot_bytes * (size_t)k1_grid));
+    const int64_t k1_base = (int64_t)ctx->num_sms * ctx->tune.tri_ctas_per_sm;
+    const TriangleSlots k1 = triangle_slots(a.cap_side, a.cap_seg, k1_grid, k1_base, ctx->slot_seg_min);
+    k1_grid = k1.grid;
+    a.slot_seg = k1.seg;
+    a.k1_slot_bytes = k1.slot_bytes;
+    CK(ctx->k1_slots.ensure(k1.bytes));
     a.k1_slots = as<char>(ctx->k1_slots);
     int64_t seg_cap = std::max<int64_t>(ctx->seg_arena.bytes / (6 * sizeof(double)), std::max<int64_t>(NP * 256, 1 << 20));
     if (plain) seg_cap = std::max<int64_t>(seg_cap, a.cap_seg);
@@ -591,7 +595,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     } else {
         a.item_begin = 0;
         a.item_end = NP;
-        for (int attempt = 0; attempt < 2; ++attempt) {
+        for (int grown = 0, whole = 0;;) {
             CK(cudaEventRecord(ctx->ev[1], st));
             launch_segments(a, k1_grid, st);
             ctx->launches += 1;
@@ -600,18 +604,33 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
             CK(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             int err = ((int*)&hc[7])[0];
-            if (!(err & ERR_SEG_ARENA)) break;
-            if (attempt == 1) return ctx_fail(ctx, ZDX_ERR_CAPACITY, "segment arena overflow after growth");
-            // grow to what the first attempt counted, then run the triangle stage again
-            int64_t need = (int64_t)hc[0] + 1024;
-            CK(ctx->seg_arena.ensure(sizeof(double) * 6 * (size_t)need));
-            a.seg = as<double>(ctx->seg_arena);
-            a.seg_cap = need;
-            if (ctx->tape_on) {
-                CK(ctx->t_segtri.ensure(sizeof(int32_t) * 2 * (size_t)need));
-                CK(ctx->t_segcand.ensure(2 * (size_t)need));
-                a.seg_tri = as<int32_t>(ctx->t_segtri);
-                a.seg_cand = as<uint8_t>(ctx->t_segcand);
+            if (whole) ctx->slot_seg_min = std::max(ctx->slot_seg_min, ((int*)&hc[6])[0]);
+            if (err & ERR_SLOT) {
+                // a pair's segments outgrew its slot: all again with whole slots, two CTAs an SM (the count of segments
+                // is short of the truth until then)
+                whole = 1;
+                const TriangleSlots w = triangle_slots(a.cap_side, a.cap_seg, std::min<int64_t>(k1_grid, k1_base), k1_base, 0);
+                k1_grid = w.grid;
+                a.slot_seg = w.seg;
+                a.k1_slot_bytes = w.slot_bytes;
+                CK(ctx->k1_slots.ensure(w.bytes));
+                a.k1_slots = as<char>(ctx->k1_slots);
+            } else if (err & ERR_SEG_ARENA) {
+                if (grown) return ctx_fail(ctx, ZDX_ERR_CAPACITY, "segment arena overflow after growth");
+                grown = 1;
+                // grow to what the first attempt counted, then run the triangle stage again
+                int64_t need = (int64_t)hc[0] + 1024;
+                CK(ctx->seg_arena.ensure(sizeof(double) * 6 * (size_t)need));
+                a.seg = as<double>(ctx->seg_arena);
+                a.seg_cap = need;
+                if (ctx->tape_on) {
+                    CK(ctx->t_segtri.ensure(sizeof(int32_t) * 2 * (size_t)need));
+                    CK(ctx->t_segcand.ensure(2 * (size_t)need));
+                    a.seg_tri = as<int32_t>(ctx->t_segtri);
+                    a.seg_cand = as<uint8_t>(ctx->t_segcand);
+                }
+            } else {
+                break;
             }
             CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * kCounters, st));
             CK(cudaMemsetAsync(a.pair_status, 0, sizeof(int32_t) * P1, st));

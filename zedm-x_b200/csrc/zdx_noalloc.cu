@@ -183,7 +183,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     a.cap_side = std::max(max_ntri, 1);
     a.flat_max = ctx->tune.flat_max;
     a.k1_threads = 256;  // the few CTAs whose slots fit want the larger block
-    a.cap_seg = seg_cap;
+    a.cap_seg = a.slot_seg = seg_cap;
     a.mesh_infl_bits = cv.take<unsigned long long>(ZDX_NOALLOC_MAX_MESHES);
     a.seg = cv.take<double>(6 * (size_t)kSegArena);
     a.seg_cap = kSegArena;

@@ -229,6 +229,31 @@ int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode) {
 int triangle_ctas(int knob, int threads) { return knob >= 2 ? (threads == 128 ? K1<128>::RESIDENT : K1<256>::RESIDENT) : 1; }
 size_t tritest_slot_bytes(int cap_side, int cap_seg) { return carve_k1(nullptr, cap_side, cap_seg, nullptr); }
 
+// A whole slot holds 16,384 segments by default, 0.95 of its 1.06 MB for meshes of 320 triangles, and the largest pairs of
+// the pair sweep have 1,800.  With whole slots for three or six CTAs an SM instead of two (base) a context held 0.96 GB
+// after 3,000 pairs of such meshes, with these 0.36.  The buffer has one size for every batch of more than base pairs: a
+// scene whose pair count climbs does not allocate it anew at each maximum (the first Scene.step of a bed of 729: 27 ms
+// with an allocation at each, 4.8 ms so).
+TriangleSlots triangle_slots(int cap_side, int cap_seg, int64_t ctas, int64_t base, int seg_min) {
+    const size_t whole = tritest_slot_bytes(cap_side, cap_seg);
+    const TriangleSlots w{(int)(ctas < base ? ctas : base), cap_seg, whole, whole * (size_t)(ctas < base ? ctas : base)};
+    if (ctas <= base) return w;
+    const size_t share = whole * (size_t)base / (size_t)ctas;
+    int seg = cap_seg < 2048 ? cap_seg : 2048;
+    if (seg < seg_min) seg = seg_min < cap_seg ? seg_min : cap_seg;
+    const size_t least = tritest_slot_bytes(cap_side, seg), one = sizeof(double) * 6 + sizeof(uint64_t) + 2;
+    if (share > least + 64) {  // 64: the roundings of its three arrays
+        const size_t more = (size_t)seg + (share - least - 64) / one;
+        seg = more < (size_t)cap_seg ? (int)more : cap_seg;
+    }
+    const size_t bytes = tritest_slot_bytes(cap_side, seg);
+    const size_t limit = whole * (size_t)base > (size_t)2 << 30 ? whole * (size_t)base : (size_t)2 << 30;
+    const int64_t fit = (int64_t)(limit / bytes), grid = ctas < fit ? ctas : fit;
+    if (grid <= base) return w;
+    const size_t total = bytes * (size_t)grid;
+    return TriangleSlots{(int)grid, seg, bytes, total > w.bytes ? total : w.bytes};
+}
+
 __device__ __forceinline__ uint32_t expand10(uint32_t v) {
     v &= 1023u;
     v = (v | (v << 16)) & 0x030000FFu;
@@ -319,7 +344,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
     const int tid = threadIdx.x;
     K1Slot S;
     char* slot = a.k1_slots + (size_t)blockIdx.x * a.k1_slot_bytes;
-    carve_k1(slot, a.cap_side, a.cap_seg, &S);
+    carve_k1(slot, a.cap_side, a.slot_seg, &S);
     const int cap = a.cap_side;
     const ptrdiff_t side_bytes = reinterpret_cast<char*>(S.side[1].tri) - reinterpret_cast<char*>(S.side[0].tri);
     const bool py = NPX || a.mode == 1;
@@ -942,7 +967,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                         }
                         if (hit) {
                             const int si = atomicAdd(&sh_nseg, 1);
-                            if (si < a.cap_seg) {
+                            if (si < a.slot_seg) {
                                 st3(S.seg + 6 * si, o0);
                                 st3(S.seg + 6 * si + 3, o1);
                                 S.key[si] = ((uint64_t)(uint32_t)S.side[0].id[e.x] << 32) | (uint64_t)(uint32_t)S.side[1].id[e.y];
@@ -984,9 +1009,10 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
         }
         int ns = sh_nseg;
         int status = 0;
-        if (ns > a.cap_seg) {
+        if (ns > a.slot_seg) {
             status |= PAIR_SEG_OVERFLOW;
-            ns = a.cap_seg;
+            ns = a.slot_seg;
+            if (a.slot_seg < a.cap_seg && tid == 0) atomicOr(a.err, ERR_SLOT);
         }
         if (tid == 0) sh_base = atomicAdd(a.seg_counter, (unsigned long long)ns);
         __syncthreads();

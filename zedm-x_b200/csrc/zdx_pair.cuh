@@ -22,6 +22,7 @@ enum : int {
     ERR_POINT_STAGE = 4,    // more loop points than loop_point_cap
     ERR_PAIR = 8,           // some pair has a non-zero status
     ERR_TAPE = 16,          // the adjoint tape arena is too small
+    ERR_SLOT = 32,          // a pair has more segments than a slot (fewer than cap_seg) holds: rerun with whole slots
 };
 
 struct PairArgs {
@@ -81,6 +82,7 @@ struct PairArgs {
     int k1_threads;  // threads of a CTA, 128 or 256 (triangle_threads)
     char* k1_slots;
     size_t k1_slot_bytes;
+    int slot_seg;  // segments a slot holds: cap_seg, or fewer (triangle_slots)
     double* seg;  // arena: 6 doubles per segment
     int64_t seg_cap;
     unsigned long long* seg_counter;  // arena entries taken (with split pairs, their temporary runs too)
@@ -194,6 +196,14 @@ size_t tritest_slot_bytes(int cap_side, int cap_seg);
 // tri_ctas_per_sm (1, or 2: as many as fit).
 int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode);
 int triangle_ctas(int knob, int threads);
+// The triangle stage's CTAs and their slots for `ctas` CTAs at most, `base` of which get slots for cap_seg segments
+// whatever they take.  More than base: slots of at least seg_min segments (2,048, or cap_seg if that is less) that
+// together take what base whole ones would, or 2 GB if that is more.
+struct TriangleSlots {
+    int grid, seg;
+    size_t slot_bytes, bytes;  // of a slot; of the buffer
+};
+TriangleSlots triangle_slots(int cap_side, int cap_seg, int64_t ctas, int64_t base, int seg_min);
 
 void launch_mesh_prep(const PairArgs& a, int64_t total_tris, cudaStream_t s);
 void launch_cost_order(const PairArgs& a, int32_t* order, int* buckets, cudaStream_t s);

@@ -1558,8 +1558,12 @@ static int graph_alloc(zdx_ctx* ctx, Scene& s) {
     CKS(G.tm_lists.ensure(sizeof(int32_t) * (TEAM_CLASSES + 1) * P1));
     // a small scene has few pairs, whatever its capacity
     G.k1_threads = s.np < kCacheMinParticles ? 256 : triangle_threads(max_ntri, (int64_t)P1, ctx->num_sms, ZDX_MODE_ZDEM);
-    G.k1_grid = (int)std::min<int64_t>(P1, (int64_t)ctx->num_sms * triangle_ctas(ctx->tune.tri_ctas_per_sm, G.k1_threads));
-    CKS(G.k1_slots.ensure(tritest_slot_bytes(max_ntri, G.cap_seg) * (size_t)G.k1_grid));
+    // whole slots: no rerun inside the captured step
+    const TriangleSlots k1 = triangle_slots(max_ntri, G.cap_seg,
+                                            std::min<int64_t>(P1, (int64_t)ctx->num_sms * triangle_ctas(ctx->tune.tri_ctas_per_sm, G.k1_threads)),
+                                            (int64_t)ctx->num_sms * ctx->tune.tri_ctas_per_sm, G.cap_seg);
+    G.k1_grid = k1.grid;
+    CKS(G.k1_slots.ensure(k1.bytes));
     CKS(G.seg_arena.ensure(sizeof(double) * 6 * (size_t)std::max<int64_t>(G.segcap, 1)));
     const size_t slot = rebuild_slot_bytes(G.cap_seg);
     int64_t warps = std::min<int64_t>((int64_t)P1, (int64_t)ctx->num_sms * 32);
@@ -1664,7 +1668,7 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         int max_ntri = 1;
         for (int m = 0; m < nm; ++m) max_ntri = std::max<int>(max_ntri, (int)(s.mesh_off[m + 1] - s.mesh_off[m]));
         a.cap_side = max_ntri;
-        a.cap_seg = G.cap_seg;
+        a.cap_seg = a.slot_seg = G.cap_seg;
         a.flat_max = ctx->tune.flat_max;
         a.k1_threads = G.k1_threads;
         const size_t P1 = (size_t)std::max<int64_t>(G.pcap, 1);
