@@ -281,6 +281,14 @@ ZDX_HD double plane_gap(V3 n, double d, V3 a, V3 b, V3 c) {
     const double lo = smin3(s0, s1, s2), hi = smax3(s0, s1, s2);
     return lo > -hi ? lo : -hi;
 }
+// What two triangles may move by, the one towards the other, and still have no segment, by their planes: gapA is how
+// far A lies beyond B's plane, gapB how far B beyond A's (plane_gap); -1: nothing.  Their distance is at least a gap less
+// what the plane's owner is off it, and at any distance above both reaches and plane_offs nothing is accepted.
+ZDX_HD double planes_clearance(double gapA, double gapB, double reachA, double reachB, double RA, double RB, double pad) {
+    if (!reaches_hold(reachA, reachB, pad)) return -1.0;
+    const double oA = plane_off(reachA, RA), oB = plane_off(reachB, RB);
+    return smax(gapA - oB, gapB - oA) - smax(reachA + oA, reachB + oB) - 8.0 * pad;
+}
 ZDX_HD bool tri_tri(const V3* A, V3 nA, double dA, const V3* B, V3 nB, double dB, V3& o0, V3& o1) {
     return tri_tri_src(A, nA, dA, B, nB, dB, o0, o1, nullptr, nullptr);
 }

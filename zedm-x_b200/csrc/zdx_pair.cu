@@ -873,10 +873,8 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
                                          slot_corner(U.tri, j, 0, cap), slot_corner(U.tri, j, 1, cap),
                                          slot_corner(U.tri, j, 2, cap));
                     };
-                    const double rA = a.tri_reach[off[0] + ta], rB = a.tri_reach[off[1] + tb];
-                    const double oA = plane_off(rA, R[0]), oB = plane_off(rB, R[1]);
-                    double clear = fmax(gap(SB, e.y, SA, e.x) - oB, gap(SA, e.x, SB, e.y) - oA) - fmax(rA + oA, rB + oB) - 8.0 * pad;
-                    if (!reaches_hold(rA, rB, pad)) clear = -1.0;
+                    const double clear = planes_clearance(gap(SB, e.y, SA, e.x), gap(SA, e.x, SB, e.y), a.tri_reach[off[0] + ta],
+                                                          a.tri_reach[off[1] + tb], R[0], R[1], pad);
                     if (clear >= tau && clear > 0.0) {
                         gmin = fminf(gmin, __double2float_rd(clear));
                     } else {
