@@ -1,5 +1,5 @@
-// Host check of the triangle stage's plane test (tri_reach, plane_off, reaches_hold, beyond_plane of zdx_math.cuh, put
-// together as k_segments does): stdin holds pairs of triangles in the mesh frame, 18 doubles as hex bit patterns each,
+// Host check of the triangle stage's plane test (tri_inflation's reach, plane_off, reaches_hold, beyond_plane of zdx_math.cuh,
+// put together as k_segments does): stdin holds pairs of triangles in the mesh frame, 18 doubles as hex bit patterns each,
 // then a pose (position and quaternion, 7 more) that both are placed by.  One line out: pairs, pairs with a segment,
 // pairs ruled out, and pairs ruled out that have one (0 expected).
 #include <cinttypes>
@@ -32,7 +32,8 @@ int main() {
         double r[2], d[2], R[2] = {0.0, 0.0};
         bool ok = true;
         for (int k = 0; k < 2; ++k) {
-            r[k] = std::nextafterf((float)tri_reach(T[k][0], T[k][1], T[k][2]), INFINITY);
+            tri_inflation(T[k][0], T[k][1], T[k][2], &r[k]);
+            r[k] = std::nextafterf((float)r[k], INFINITY);
             for (int i = 0; i < 3; ++i) {
                 R[k] = smax(R[k], norm(T[k][i]));
                 T[k][i] = qrotate_n(q, T[k][i]) + x;

@@ -45,7 +45,8 @@ int main() {
                 R[k] = smax(R[k], norm(L[k][i]) * (1.0 + 1e-12));
                 T[k][i] = qrotate_n(q[k], L[k][i]) + x[k];
             }
-            r[k] = std::nextafterf((float)tri_reach(L[k][0], L[k][1], L[k][2]), INFINITY);
+            tri_inflation(L[k][0], L[k][1], L[k][2], &r[k]);
+            r[k] = std::nextafterf((float)r[k], INFINITY);
             ok = plane_from_tri(T[k][0], T[k][1], T[k][2], nn[k], d[k]) && ok;
         }
         if (!ok) continue;

@@ -23,7 +23,7 @@ def _call(ctx, lib, pm, pp, mode, split, tol):
 def test_every_class_holds_its_pairs(ctx, mode, split, tol):
     lib, pm, pp = _batch()
     n = _call(ctx, lib, pm, pp, mode, split, tol)[0]["stats"][:, 0]
-    # pairs without segments are settled where the classes are made, so nothing can be refused here
+    # pairs without segments are settled where the classes are made: no class is launched, and nothing can be refused
     apart = pp.copy()
     apart[:, 7:10] += 1.0
     r, base = _call(ctx, lib, pm, apart, mode, split, tol)
@@ -33,9 +33,9 @@ def test_every_class_holds_its_pairs(ctx, mode, split, tol):
         assert len(sel) >= 12
         # together, in packs, and the largest of the class alone
         for some in (sel, sel[np.argsort(-n[sel])][:1]):
-            assert _call(ctx, lib, pm[some], pp[some], mode, split, tol)[1] == base + c, (lo, hi, len(some))
+            assert _call(ctx, lib, pm[some], pp[some], mode, split, tol)[1] == base + 1 + c, (lo, hi, len(some))
     sel = np.nonzero(n <= CLASS_ENDS[-1])[0]
-    assert _call(ctx, lib, pm[sel], pp[sel], mode, split, tol)[1] == base + len(CLASS_ENDS) - 1
+    assert _call(ctx, lib, pm[sel], pp[sel], mode, split, tol)[1] == base + len(CLASS_ENDS)
     # and above the last class the warp form is launched
     over = np.nonzero(n > CLASS_ENDS[-1])[0][:1]
-    assert _call(ctx, lib, pm[over], pp[over], mode, split, tol)[1] == base + len(CLASS_ENDS)
+    assert _call(ctx, lib, pm[over], pp[over], mode, split, tol)[1] == base + len(CLASS_ENDS) + 1

@@ -638,7 +638,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
         }
         // stage 2: rebuild, by teams in shared memory; the pairs no team holds and every pair of the plain
         // per-stage form one warp per pair, slots sized for the largest pair
-        const int nmax = std::max(((int*)&hc[6])[0], 1);
+        const int most_seg = ((int*)&hc[6])[0], nmax = std::max(most_seg, 1);
         const size_t budget = (size_t)2 << 30;
         auto warp_form = [&](const int32_t* order, const int64_t pairs) -> int {
             a.k2_nmax = nmax;
@@ -671,11 +671,11 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
             int st_code = rebuild_by_arenas(ctx, a, NP, nmax, budget, st);
             if (st_code != ZDX_OK) return st_code;
         } else if (teams) {
-            const bool fork = team_classes_of(nmax) > 1;
+            const bool fork = team_classes_of(most_seg) > 1;
             if (fork)
                 if (int rc = second_stream(ctx)) return rc;
             const TeamSide side{ctx->stream2, {ctx->ev2[0], ctx->ev2[1]}};
-            ctx->launches += launch_rebuild_teams(a, plan, ctx->num_sms, NP, nmax, st, fork ? &side : nullptr);
+            ctx->launches += launch_rebuild_teams(a, plan, ctx->num_sms, NP, most_seg, st, fork ? &side : nullptr);
         } else {
             int st_code = warp_form(a.order, NP);
             if (st_code != ZDX_OK) return st_code;

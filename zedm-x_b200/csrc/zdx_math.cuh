@@ -234,7 +234,12 @@ ZDX_HD bool tri_join(V3 nA, V3 nB, unsigned valid, const Pt& pt, V3& o0, V3& o1,
 // How far outside triangle (p0, p1, p2) point_in_tri can accept a point: it accepts c_k = |e_k| x (in-plane distance
 // to edge line k) >= -1e-10, so each edge line moves out by 1e-10 / |e_k| and a vertex by at most
 // 2 max_k(1e-10 / |e_k|) / sin(its angle).
-ZDX_HD double tri_inflation(V3 p0, V3 p1, V3 p2) {
+//
+// And *reach: the same for the plane tests below, with the rounding of point_in_tri's products added to its 1e-10.  The
+// cross product is off by some eps l^2 (l: the longest edge), which tilts the normal of a thin triangle by eps l^2 over
+// twice its area; where that is no small angle its plane says nothing about the triangle: infinite.  (64 eps covers the
+// products, the differences and a rotation's roundings.)
+ZDX_HD double tri_inflation(V3 p0, V3 p1, V3 p2, double* reach) {
     const V3 e0 = p1 - p0, e1 = p2 - p1, e2 = p0 - p2;
     const double l0 = norm(e0), l1 = norm(e1), l2 = norm(e2);
     const double cr = norm(cross(e0, e2));
@@ -242,19 +247,13 @@ ZDX_HD double tri_inflation(V3 p0, V3 p1, V3 p2) {
     const double dmax = 1e-10 / smin3(l0, l1, l2);
     double infl = 2.0 * dmax / smin_ang;
     if (!(infl < 1e300)) infl = 1e300;
+    const double l = smax3(l0, l1, l2), round = 64.0 * 2.220446049250313e-16 * l * l;
+    *reach = round < 0.01 * cr ? 1.001 * infl * (1.0 + 1e10 * round) : __builtin_huge_val();
     return infl * (1.0 + 1e-6);
 }
-// How far outside a triangle, along its computed plane, the exact tests may accept a point, for the plane tests below:
-// tri_inflation with the rounding of point_in_tri's products added to its 1e-10.  The cross product is off by some eps l^2
-// (l: the longest edge), which tilts the normal of a thin triangle by eps l^2 over twice its area; where that is no small
-// angle its plane says nothing about the triangle: infinite.  (64 eps covers the products, the differences and a
-// rotation's roundings.)
-ZDX_HD double tri_reach(V3 p0, V3 p1, V3 p2) {
-    const V3 e0 = p1 - p0, e1 = p2 - p1, e2 = p0 - p2;
-    const double l = smax3(norm(e0), norm(e1), norm(e2));
-    const double round = 64.0 * 2.220446049250313e-16 * l * l;
-    if (!(round / norm(cross(e0, e2)) < 0.01)) return __builtin_huge_val();
-    return 1.001 * tri_inflation(p0, p1, p2) * (1.0 + 1e10 * round);
+ZDX_HD double tri_inflation(V3 p0, V3 p1, V3 p2) {
+    double reach;
+    return tri_inflation(p0, p1, p2, &reach);
 }
 // How far a triangle's own corners can stand off its computed plane, from its reach and the radius R of its mesh:
 // by the tilt times l, 64 eps l^3 / (2 area), which is at most 7.2e-5 l^2 of the reach (2e-10 l^2 / (2 area l) and

@@ -84,8 +84,9 @@ __global__ void k_mesh_prep(PairArgs a, int64_t total) {
         valid = !(norm(cross(p1 - p0, p2 - p0)) < 1e-30) ? 1 : 0;
         if (a.tri_reach && !valid) a.tri_reach[t] = __int_as_float(0x7f800000);
         if (a.mesh_infl_bits && valid) {
-            ib = (unsigned long long)__double_as_longlong(tri_inflation(p0, p1, p2));
-            if (a.tri_reach) a.tri_reach[t] = __double2float_ru(zdx::tri_reach(p0, p1, p2));
+            double reach;
+            ib = (unsigned long long)__double_as_longlong(tri_inflation(p0, p1, p2, &reach));
+            if (a.tri_reach) a.tri_reach[t] = __double2float_ru(reach);
         }
     }
     // A mesh's triangles are consecutive, so they are runs of lanes: reduce each run (max, sum, max of
@@ -222,7 +223,9 @@ __host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, K1S
 // Meshes of up to 1,280 triangles leave a block of 256 half idle in most of a pair's phases: blocks of 128, twice as
 // many, take 0.74 against 0.95 ms on 16,384 pairs of 320-triangle meshes, 26.9 against 28.3 ms for ten steps of a
 // 30,000-particle pour (124 to 1,280 triangles), and 1.55 against 1.23 ms on 1,500 pairs of 5,120.  A batch that
-// gives an SM less than six pairs wants the larger block for each (64 mixed pairs: 0.26 against 0.50 ms).
+// gives an SM less than six pairs wants the larger block for each (64 mixed pairs: 0.26 against 0.50 ms).  Meshes
+// between 1,280 and 5,120 triangles were not timed, and the largest mesh of the set decides, whether a pair uses it or
+// not.
 int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode) {
     return mode != 2 && max_ntri <= 1280 && pairs >= 6 * (int64_t)sms ? 128 : 256;
 }

@@ -34,7 +34,7 @@ struct PairArgs {
     const double* bbox_diag;
     // per-triangle bounding spheres (cx, cy, cz, r) in the mesh frame and per-mesh bounds (k_mesh_prep)
     double4* tri_sph;
-    // per triangle, how far outside it a point may be accepted (zdx::tri_reach, rounded up; k_mesh_prep); null with
+    // per triangle, how far outside it a point may be accepted (tri_inflation's reach, rounded up; k_mesh_prep); null with
     // mesh_infl_bits
     float* tri_reach;
     unsigned long long* mesh_R_bits;  // max over triangles of |c| + r, as the bits of a positive double
@@ -134,7 +134,8 @@ struct PairArgs {
     // vertex of B by mu_B with mu_A + mu_B < M (less the rounding allowance); the near pairs are tested
     // again.  cache_idx[p] >= 0 names the entry of cache_in found for pair p, which k_segments uses to
     // skip the pair while it holds; cache_out / cache_hout receive each pair's entry for the next step
-    // (M <= 0: none).  cache_tau (times R_A + R_B) is the box gap below which a survivor pair is near.
+    // (M <= 0: none).  A survivor pair is near when neither its boxes nor one triangle's plane hold it apart
+    // by cache_tau (times R_A + R_B).
     const int32_t* cache_idx;
     const double* cache_in;
     double* cache_out;
@@ -208,8 +209,8 @@ TriangleSlots triangle_slots(int cap_side, int cap_seg, int64_t ctas, int64_t ba
 void launch_mesh_prep(const PairArgs& a, int64_t total_tris, cudaStream_t s);
 void launch_cost_order(const PairArgs& a, int32_t* order, int* buckets, cudaStream_t s);
 void launch_segments(const PairArgs& a, int grid, cudaStream_t s);
-// The clearance cache's skips, before the cost order: a warp per pair with an entry tests its motion
-// against the clearance and its near pairs again; a pair settled so gets the outputs of a pair without
+// The clearance cache's skips, before the cost order: a warp per up to 16 pairs tests the motion of those with an
+// entry against the clearance and their near pairs again; a pair settled so gets the outputs of a pair without
 // segments (triangle stage and rebuild), its entry carried over, and cache_skip[p] = 1.
 void launch_cache_skip(const PairArgs& a, int grid, cudaStream_t s);
 void launch_rebuild(const PairArgs& a, int warps, int warps_per_block, cudaStream_t s);

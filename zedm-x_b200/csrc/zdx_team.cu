@@ -28,8 +28,10 @@ struct TeamClass {
     int bytes;     // shared memory of a block
     int threads;
 };
-// A pair needs about 150 bytes a segment (205 at most over the pair sweep's mesh sizes).  The lines lie where the
-// next larger memory would cost a resident block: three, two and one an SM.
+// A pair needs about 150 bytes a segment (205 at most over the pair sweep's mesh sizes; the memories hold 217, 195 and 195
+// at the lines, so the top of the larger classes may go to the warp form: none did among pairs of all six modes and
+// settings of the tests).  The lines lie where the next larger memory would cost a resident block: three, two and one an
+// SM.
 __host__ __device__ constexpr TeamClass team_class(int c) {
     return c == 0   ? TeamClass{330, 380, 70 * 1024, 256}
            : c == 1 ? TeamClass{560, 560, 107 * 1024, 256}
@@ -167,7 +169,7 @@ int launch_classes(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most,
     }
     if (n > 2) launch_class<2, 1, NPX>(a, pl, sms, most, s2);
     if (n > 1) launch_class<1, 2, NPX>(a, pl, sms, most, s2);
-    launch_class<0, 3, NPX>(a, pl, sms, most, s);
+    if (n > 0) launch_class<0, 3, NPX>(a, pl, sms, most, s);  // none: no pair has a segment
     if (side) {
         cudaEventRecord(side->ev[1], s2);
         cudaStreamWaitEvent(s, side->ev[1], 0);
@@ -177,7 +179,7 @@ int launch_classes(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most,
 
 }  // namespace
 
-int team_classes_of(int nmax) { return nmax <= team_class(0).max_seg ? 1 : nmax <= team_class(1).max_seg ? 2 : 3; }
+int team_classes_of(int nmax) { return nmax <= 0 ? 0 : nmax <= team_class(0).max_seg ? 1 : nmax <= team_class(1).max_seg ? 2 : 3; }
 
 int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s,
                          const TeamSide* side) {
