@@ -261,10 +261,12 @@ int zdx_scene_step_graph(zdx_ctx* ctx, int nsteps);
 int zdx_scene_graph_reserve(zdx_ctx* ctx, int64_t pairs, int64_t contacts, int64_t segments, int seg_per_pair);
 /* The graph step's clearance cache (no reference counterpart; config key contact_cache, default 1; in
  * scenes of 256 particles or more): a candidate pair whose triangle stage found no segment keeps a
- * clearance M with the two poses and its near triangle pairs (boxes closer than contact_cache_tau x
- * (R_A + R_B)); while the vertices of the two bodies have moved by at most mu_A + mu_B < M since
+ * clearance M with the two poses and its near triangle pairs (those that neither their boxes nor one
+ * triangle's plane hold contact_cache_tau x (R_A + R_B) apart; a margin that is not positive counts as
+ * 0); while the vertices of the two bodies have moved by at most mu_A + mu_B < M since
  * (mu <= |x - x0| + 2 R min(|q - q0|, |q + q0|), R the mesh's bounding radius) and none of the near
- * pairs meets, the pair is known to have no segment and its triangle stage is skipped.  Results are those of the step without the cache, bit for bit.
+ * pairs meets, the pair is known to have no segment and its triangle stage is skipped.  Results are those
+ * of the step without the cache, bit for bit.
  * *entries: the cache's entries after the last graph step; *skipped: the pairs that step skipped. */
 int zdx_scene_graph_cache(zdx_ctx* ctx, int64_t* entries, int64_t* skipped);
 /* The whole zdem_cpu run after argument parsing (src/main.cpp:1879-2503) on CUDA device `device`:
@@ -392,7 +394,8 @@ int zdx_broad_phase(zdx_ctx* ctx, const double* state, const double* mat, int32_
  *     reserving a pool that takes the rest of the device, and before any stream capture.
  *   - Triangle-stage CTAs and rebuild warps share what the fixed buffers leave of the array (7.9 MiB):
  *     their slots are sized for the call's largest mesh and largest segment count, so calls on small
- *     meshes run on more CTAs and warps (4 triangle-stage CTAs at 5120 triangles, 18 at 1280, 51 at 320).
+ *     meshes run on more CTAs and warps (6 triangle-stage CTAs at 5120 triangles, 17 at 1280, 51 at 320; the
+ *     rebuild takes warps for the pairs alone that blocks in shared memory do not hold).
  *   - Every call on a device shares the one array and leaves its contents there (what must start at zero
  *     is cleared by each call); calls that overlap on the GPU race on it. */
 #define ZDX_NOALLOC_SCRATCH_BYTES (16u << 20)

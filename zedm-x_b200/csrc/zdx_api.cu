@@ -525,6 +525,7 @@ extern "C" int zdx_pair_contacts(zdx_ctx* ctx, const zdx_pair_opts* opts, const 
     const TriangleSlots k1 = triangle_slots(a.cap_side, a.cap_seg, k1_grid, k1_base, ctx->slot_seg_min);
     k1_grid = k1.grid;
     a.slot_seg = k1.seg;
+    a.cap_list = triangle_list_cap(a.cap_side);
     a.k1_slot_bytes = k1.slot_bytes;
     CK(ctx->k1_slots.ensure(k1.bytes));
     a.k1_slots = as<char>(ctx->k1_slots);

@@ -55,6 +55,7 @@ struct zdx_ctx {
     zdx::DevBuf tri_sph, mesh_R, mesh_valid, mesh_infl;
     zdx::DevBuf order, buckets, pair_i64, pair_i32, counters;
     zdx::DevBuf k1_slots, seg_arena, k2_slots;
+    bool noalloc_loaded = false;  // zdx_pair_contacts_noalloc has loaded every kernel it may launch
     int slot_seg_min = 0;  // segments a triangle-stage slot must hold: the most that a rerun with whole slots met
     zdx::DevBuf tm_lists;                        // team form of the rebuild: class lists
     zdx::DevBuf ar_lists, ar_counts, ar_gslots;  // arena form of the rebuild: class lists, counts, slots

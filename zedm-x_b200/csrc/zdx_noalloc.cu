@@ -30,6 +30,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[ZDX_NOALLOC_SCR
 
 constexpr int kMaxDevices = 128;
 constexpr int kSegArena = 65536;   // segments per call
+constexpr int kCounters = 16 + TEAM_COUNTS / 2;  // the call's, then the team rebuild's
 
 std::mutex g_mu;
 unsigned char* g_scratch_addr[kMaxDevices] = {};
@@ -145,6 +146,12 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     unsigned char* base = nullptr;
     int rc = scratch_address(ctx, &base);
     if (rc) return rc;
+    if (!ctx->noalloc_loaded) {
+        // the code of the rebuild's kernels, of which a call runs those its pairs need: loading takes device memory
+        CKN(load_rebuild_teams());
+        CKN(load_rebuild());
+        ctx->noalloc_loaded = true;
+    }
 
     // carve the scratch array
     const size_t P1 = (size_t)std::max<int64_t>(NP, 1);
@@ -156,7 +163,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     a.mean_edge = ms->mean_edge;
     a.bbox_diag = ms->bbox_diag;
     a.tri_sph = cv.take<double4>(ZDX_NOALLOC_MAX_TRIS);
-    a.tri_reach = cv.take<float>(ZDX_NOALLOC_MAX_TRIS);
+    a.tri_reach = cv.take<float>((size_t)total_tris);
     a.mesh_R_bits = cv.take<unsigned long long>(ZDX_NOALLOC_MAX_MESHES);
     a.mesh_valid = cv.take<int>(ZDX_NOALLOC_MAX_MESHES);
     a.n_pairs = NP;
@@ -169,7 +176,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     a.tol_in = opts->mode == ZDX_MODE_POLYLINE ? (opts->tol > 0.0 ? opts->tol : 1e-6) : opts->tol;
     a.k = opts->k;
     a.want_pts = 0;
-    unsigned long long* cnt = cv.take<unsigned long long>(16);
+    unsigned long long* cnt = cv.take<unsigned long long>(kCounters);
     a.seg_counter = cnt + 0;
     a.contact_counter = cnt + 1;
     a.pts_counter = cnt + 2;
@@ -183,7 +190,13 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     a.cap_side = std::max(max_ntri, 1);
     a.flat_max = ctx->tune.flat_max;
     a.k1_threads = 256;  // the few CTAs whose slots fit want the larger block
-    a.cap_seg = a.slot_seg = seg_cap;
+    a.cap_seg = seg_cap;
+    // Slots as small as they can be, so that more CTAs fit: no pair has more segments than triangle pairs, and lists of six
+    // entries a triangle take no more than the boxes that slots held before the lists.  With lists of 1,024 entries at
+    // least, and a warp a pair in the rebuild, 4,000 pairs of 20-triangle meshes took 0.47 ms where slots with boxes had
+    // taken 0.40, of 80 1.08 and 0.94, 1,500 of 320 1.68 and 1.55; so 0.31, 0.75 and 0.79.
+    a.slot_seg = (int)std::min<int64_t>(seg_cap, (int64_t)a.cap_side * a.cap_side);
+    a.cap_list = std::min(triangle_list_cap(a.cap_side), std::max(6 * a.cap_side, 16));
     a.mesh_infl_bits = cv.take<unsigned long long>(ZDX_NOALLOC_MAX_MESHES);
     a.seg = cv.take<double>(6 * (size_t)kSegArena);
     a.seg_cap = kSegArena;
@@ -204,6 +217,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     a.pts_stage = nullptr;
     a.pts_cap = 0;
     int64_t* poff = cv.take<int64_t>(ZDX_NOALLOC_MAX_PAIRS + 1);
+    const TeamPlan plan{cv.take<int32_t>((TEAM_CLASSES + 1) * P1), (int64_t)P1, reinterpret_cast<int*>(cnt + 16)};
     // The rest of the array holds the per-CTA slots of the triangle stage and, once that stage is done,
     // the per-warp slots of the rebuild stage (the same bytes; the stream orders the two).  Slots are
     // sized for this call's largest mesh and, after the triangle stage, for its largest segment count,
@@ -213,7 +227,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
         return ctx_fail(ctx, ZDX_ERR_INVALID, "noalloc scratch layout needs %zu bytes", var_off);
     const size_t room = ZDX_NOALLOC_SCRATCH_BYTES - var_off;
     char* var_base = reinterpret_cast<char*>(base + var_off);
-    a.k1_slot_bytes = (tritest_slot_bytes(a.cap_side, seg_cap) + 255) & ~size_t(255);
+    a.k1_slot_bytes = (tritest_slot_bytes(a.cap_side, a.slot_seg, a.cap_list) + 255) & ~size_t(255);
     const int64_t k1_fit = (int64_t)(room / a.k1_slot_bytes);
     if (k1_fit < 1) return ctx_fail(ctx, ZDX_ERR_INVALID, "noalloc call: a triangle-stage slot does not fit the scratch array");
     const int k1_grid = (int)std::min<int64_t>(std::min<int64_t>(k1_fit, (int64_t)ctx->num_sms * triangle_ctas(ctx->tune.tri_ctas_per_sm, a.k1_threads)),
@@ -222,7 +236,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
 
     // clear what must start at zero; everything else is written before it is read
     CKN(cudaEventRecord(ctx->ev[0], st));
-    CKN(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 16, st));
+    CKN(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * kCounters, st));
     CKN(cudaMemsetAsync(a.pair_status, 0, sizeof(int32_t) * P1, st));
     CKN(cudaMemsetAsync(a.mesh_R_bits, 0, sizeof(unsigned long long) * std::max(NM, 1), st));
     CKN(cudaMemsetAsync(a.mesh_valid, 0, sizeof(int) * std::max(NM, 1), st));
@@ -233,7 +247,7 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
     CKN(cudaGetLastError());
     ctx->launches += total_tris > 0 ? 1 : 0;
     ctx->launches += NP > 0 ? 3 : 0;
-    unsigned long long hc[8];
+    unsigned long long hc[kCounters];
     if (NP > 0) {
         launch_segments(a, k1_grid, st);
         ctx->launches += 1;
@@ -242,20 +256,35 @@ extern "C" int zdx_pair_contacts_noalloc(zdx_ctx* ctx, const zdx_pair_opts* opts
         CKN(cudaStreamSynchronize(st));
         if (static_cast<int>(hc[7] & 0xffffffffull) & ERR_SEG_ARENA)
             return ctx_fail(ctx, ZDX_ERR_CAPACITY, "noalloc call: more than %d segments in one call", kSegArena);
-        a.k2_nmax = std::max(static_cast<int>(hc[6] & 0xffffffffull), 1);
-        a.k2_slot_bytes = (rebuild_slot_bytes(a.k2_nmax) + 255) & ~size_t(255);
-        const int64_t k2_fit = (int64_t)(room / a.k2_slot_bytes);
-        if (k2_fit < 1)
-            return ctx_fail(ctx, ZDX_ERR_INVALID, "noalloc call: a rebuild slot for %d segments does not fit the scratch array",
-                            a.k2_nmax);
-        a.k2_nslots = std::min<int64_t>(std::min<int64_t>(k2_fit, (int64_t)ctx->num_sms * 32), NP);
-        a.k2_slots = var_base;
-        launch_rebuild(a, (int)a.k2_nslots, ctx->tune.rebuild_warps, st);
-        ctx->launches += 1;
+        // the rebuild by teams, on this stream alone; the pairs no team holds by a warp each
+        const int most_seg = static_cast<int>(hc[6] & 0xffffffffull);
+        ctx->launches += launch_rebuild_teams(a, plan, ctx->num_sms, NP, most_seg, st);
         CKN(cudaGetLastError());
+        CKN(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
+        CKN(cudaStreamSynchronize(st));
+        const int left = reinterpret_cast<int*>(hc + 16)[TEAM_CLASSES];
+        if (left > 0) {
+            a.k2_nmax = std::max(most_seg, 1);
+            a.k2_slot_bytes = (rebuild_slot_bytes(a.k2_nmax) + 255) & ~size_t(255);
+            const int64_t k2_fit = (int64_t)(room / a.k2_slot_bytes);
+            if (k2_fit < 1)
+                return ctx_fail(ctx, ZDX_ERR_INVALID, "noalloc call: a rebuild slot for %d segments does not fit the scratch array",
+                                a.k2_nmax);
+            a.k2_nslots = std::min<int64_t>(std::min<int64_t>(k2_fit, (int64_t)ctx->num_sms * 32), left);
+            a.k2_slots = var_base;
+            PairArgs w = a;
+            w.order = plan.lists + TEAM_CLASSES * plan.stride;
+            w.item_end = left;
+            launch_rebuild(w, (int)a.k2_nslots, ctx->tune.rebuild_warps, st);
+            ctx->launches += 1;
+            CKN(cudaGetLastError());
+            CKN(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
+            CKN(cudaStreamSynchronize(st));
+        }
+    } else {
+        CKN(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
+        CKN(cudaStreamSynchronize(st));
     }
-    CKN(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
-    CKN(cudaStreamSynchronize(st));
     const int err = static_cast<int>(hc[7] & 0xffffffffull);
     out->totals[0] = (int64_t)hc[1];
     out->totals[1] = (int64_t)hc[0];

@@ -45,8 +45,9 @@ struct K1 {
     // (64 registers) 10.8.
     static constexpr int RESIDENT = 768 / T;
 };
-// Entries of a CTA's two lists of triangle pairs (boxes that overlap; those the plane test leaves).
-__host__ __device__ inline int k1_list_cap(int cap) {
+// Entries of a CTA's two lists of triangle pairs (boxes that overlap; those the plane test leaves); pairs with more
+// are taken in windows.
+int triangle_list_cap(int cap) {
     const int n = 8 * cap;
     return n < 1024 ? 1024 : (n > 8192 ? 8192 : n);
 }
@@ -185,13 +186,13 @@ struct K1Side {
 };
 struct K1Slot {
     K1Side side[2];
-    uint2* list[2];  // k1_list_cap(cap): triangle pairs (A survivor, B survivor)
+    uint2* list[2];  // cap_list: triangle pairs (A survivor, B survivor)
     double* seg;    // 6 x cap_seg
     uint64_t* key;  // cap_seg
     uint8_t* cand;  // 2 x cap_seg: candidate index of each endpoint (adjoint tape)
 };
 
-__host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, K1Slot* s) {
+__host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, int cap_list, K1Slot* s) {
     size_t off = 0;
     auto take = [&](size_t bytes) -> char* {
         char* p = base ? base + off : nullptr;
@@ -203,7 +204,7 @@ __host__ __device__ inline size_t carve_k1(char* base, int cap, int cap_seg, K1S
         d.tri = (double*)take(sizeof(double) * 9 * (size_t)cap);
         d.pl = (double*)take(sizeof(double) * 4 * (size_t)cap);
         d.id = (int*)take(sizeof(int) * (size_t)cap);
-        uint2* l = (uint2*)take(sizeof(uint2) * (size_t)k1_list_cap(cap));
+        uint2* l = (uint2*)take(sizeof(uint2) * (size_t)cap_list);
         if (s) {
             s->side[k] = d;
             s->list[k] = l;
@@ -230,7 +231,9 @@ int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode) {
     return mode != 2 && max_ntri <= 1280 && pairs >= 6 * (int64_t)sms ? 128 : 256;
 }
 int triangle_ctas(int knob, int threads) { return knob >= 2 ? (threads == 128 ? K1<128>::RESIDENT : K1<256>::RESIDENT) : 1; }
-size_t tritest_slot_bytes(int cap_side, int cap_seg) { return carve_k1(nullptr, cap_side, cap_seg, nullptr); }
+size_t tritest_slot_bytes(int cap_side, int cap_seg, int cap_list) {
+    return carve_k1(nullptr, cap_side, cap_seg, cap_list, nullptr);
+}
 
 // A whole slot holds 16,384 segments by default, 0.95 of its 1.06 MB for meshes of 320 triangles, and the largest pairs of
 // the pair sweep have 1,800.  With whole slots for three or six CTAs an SM instead of two (base) a context held 0.96 GB
@@ -238,18 +241,19 @@ size_t tritest_slot_bytes(int cap_side, int cap_seg) { return carve_k1(nullptr, 
 // scene whose pair count climbs does not allocate it anew at each maximum (the first Scene.step of a bed of 729: 27 ms
 // with an allocation at each, 4.8 ms so).
 TriangleSlots triangle_slots(int cap_side, int cap_seg, int64_t ctas, int64_t base, int seg_min) {
-    const size_t whole = tritest_slot_bytes(cap_side, cap_seg);
+    const int list = triangle_list_cap(cap_side);
+    const size_t whole = tritest_slot_bytes(cap_side, cap_seg, list);
     const TriangleSlots w{(int)(ctas < base ? ctas : base), cap_seg, whole, whole * (size_t)(ctas < base ? ctas : base)};
     if (ctas <= base) return w;
     const size_t share = whole * (size_t)base / (size_t)ctas;
     int seg = cap_seg < 2048 ? cap_seg : 2048;
     if (seg < seg_min) seg = seg_min < cap_seg ? seg_min : cap_seg;
-    const size_t least = tritest_slot_bytes(cap_side, seg), one = sizeof(double) * 6 + sizeof(uint64_t) + 2;
+    const size_t least = tritest_slot_bytes(cap_side, seg, list), one = sizeof(double) * 6 + sizeof(uint64_t) + 2;
     if (share > least + 64) {  // 64: the roundings of its three arrays
         const size_t more = (size_t)seg + (share - least - 64) / one;
         seg = more < (size_t)cap_seg ? (int)more : cap_seg;
     }
-    const size_t bytes = tritest_slot_bytes(cap_side, seg);
+    const size_t bytes = tritest_slot_bytes(cap_side, seg, list);
     const size_t limit = whole * (size_t)base > (size_t)2 << 30 ? whole * (size_t)base : (size_t)2 << 30;
     const int64_t fit = (int64_t)(limit / bytes), grid = ctas < fit ? ctas : fit;
     if (grid <= base) return w;
@@ -347,7 +351,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
     const int tid = threadIdx.x;
     K1Slot S;
     char* slot = a.k1_slots + (size_t)blockIdx.x * a.k1_slot_bytes;
-    carve_k1(slot, a.cap_side, a.slot_seg, &S);
+    carve_k1(slot, a.cap_side, a.slot_seg, a.cap_list, &S);
     const int cap = a.cap_side;
     const ptrdiff_t side_bytes = reinterpret_cast<char*>(S.side[1].tri) - reinterpret_cast<char*>(S.side[0].tri);
     const bool py = NPX || a.mode == 1;
@@ -682,7 +686,7 @@ __global__ __launch_bounds__(T, K1<T>::RESIDENT) void k_segments(PairArgs a) {
         const int nA = near_only ? 0 : sh_n[0], nB = near_only ? 0 : sh_n[1];
         const K1Side& SA = S.side[0];
         const K1Side& SB = S.side[1];
-        const int lcap = k1_list_cap(cap);
+        const int lcap = a.cap_list;
         const int lane = tid & 31, warp = tid >> 5;
         // the reference's AABB reject (src/main.cpp:2130-2134), strict compares; all six at once, as a chain of
         // short-circuits waits out a load for each
@@ -2184,6 +2188,11 @@ void launch_rebuild(const PairArgs& a, int warps, int warps_per_block, cudaStrea
         cudaFuncSetAttribute(k_rebuild<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
         k_rebuild<false><<<blocks, wpb * 32, 0, s>>>(a);
     }
+}
+
+cudaError_t load_rebuild() {
+    cudaFuncAttributes f;
+    return cudaFuncGetAttributes(&f, k_rebuild<false>);
 }
 
 // --------------------------------------------------------------------------------------------- stage 3

@@ -83,6 +83,7 @@ struct PairArgs {
     char* k1_slots;
     size_t k1_slot_bytes;
     int slot_seg;  // segments a slot holds: cap_seg, or fewer (triangle_slots)
+    int cap_list;  // entries of a slot's lists of triangle pairs (triangle_list_cap)
     double* seg;  // arena: 6 doubles per segment
     int64_t seg_cap;
     unsigned long long* seg_counter;  // arena entries taken (with split pairs, their temporary runs too)
@@ -191,8 +192,10 @@ struct TeamSide {
 int team_classes_of(int nmax);  // classes that pairs of up to nmax segments take
 int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t most, int nmax, cudaStream_t s,
                          const TeamSide* side = nullptr);
-// Bytes of one triangle-stage slot.
-size_t tritest_slot_bytes(int cap_side, int cap_seg);
+cudaError_t load_rebuild_teams();  // loads the code of every class (but numpy mode's)
+// Bytes of one triangle-stage slot, and the entries of its lists unless there is no room for them.
+size_t tritest_slot_bytes(int cap_side, int cap_seg, int cap_list);
+int triangle_list_cap(int cap_side);
 // Threads of a triangle-stage CTA for a batch (PairArgs::k1_threads), and the CTAs an SM runs for the tuning value
 // tri_ctas_per_sm (1, or 2: as many as fit).
 int triangle_threads(int max_ntri, int64_t pairs, int sms, int mode);
@@ -214,6 +217,7 @@ void launch_segments(const PairArgs& a, int grid, cudaStream_t s);
 // segments (triangle stage and rebuild), its entry carried over, and cache_skip[p] = 1.
 void launch_cache_skip(const PairArgs& a, int grid, cudaStream_t s);
 void launch_rebuild(const PairArgs& a, int warps, int warps_per_block, cudaStream_t s);
+cudaError_t load_rebuild();  // loads its code (but numpy mode's)
 void launch_gather(const PairArgs& a, int64_t* pair_contact_off, int64_t* pair_pts_off, double* cgeom,
                    int32_t* cinfo, double* pts, int64_t* cpt_off, int32_t* pair_stats, int64_t* ctape_off,
                    cudaStream_t s);

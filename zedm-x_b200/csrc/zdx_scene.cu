@@ -1713,7 +1713,8 @@ static int graph_launch_step(zdx_ctx* ctx, Scene& s) {
         a.order = as<int32_t>(G.order);
         a.item_begin = 0;
         a.item_end = G.pcap;
-        a.k1_slot_bytes = tritest_slot_bytes(a.cap_side, a.cap_seg);
+        a.cap_list = triangle_list_cap(a.cap_side);
+        a.k1_slot_bytes = tritest_slot_bytes(a.cap_side, a.cap_seg, a.cap_list);
         a.k1_slots = as<char>(G.k1_slots);
         a.seg = as<double>(G.seg_arena);
         a.seg_cap = G.segcap;

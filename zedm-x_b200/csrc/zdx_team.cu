@@ -189,4 +189,14 @@ int launch_rebuild_teams(const PairArgs& a, const TeamPlan& pl, int sms, int64_t
                             : launch_classes<false>(a, pl, sms, most, nmax, s, side));
 }
 
+cudaError_t load_rebuild_teams() {
+    cudaFuncAttributes f;
+    const void* ks[4] = {(const void*)k_team_classes, (const void*)k_rebuild_team<team_class(0).threads, 3, false>,
+                         (const void*)k_rebuild_team<team_class(1).threads, 2, false>,
+                         (const void*)k_rebuild_team<team_class(2).threads, 1, false>};
+    for (const void* k : ks)
+        if (cudaError_t e = cudaFuncGetAttributes(&f, k)) return e;
+    return cudaSuccess;
+}
+
 }  // namespace zdx
