@@ -180,7 +180,7 @@ def measured_peaks():
 PROFILED = {
     "sources_sha256": "558857edb9ac4f06dffda0ce39fe3ef15e9349423a04fe370a57d4fced13788b",
     "k_segments": {"warp_inst_per_pair": 82215.3, "dram_bytes_per_pair": 140241.2},
-    "k_rebuild": {"warp_inst_per_pair": 63880.8, "dram_bytes_per_pair": 5259.2},  # the team kernels, all classes
+    "k_rebuild_team": {"warp_inst_per_pair": 63880.8, "dram_bytes_per_pair": 5259.2},  # all classes
 }
 KERNEL_SOURCES = ("zdx_pair.cu", "zdx_pair.cuh", "zdx_math.cuh", "zdx_npmath.cuh", "zdx_pyset.cuh",
                   "zdx_sortrep.cuh", "zdx_radix.cuh", "zdx_team.cu", "zdx_team.cuh")
@@ -215,7 +215,7 @@ def issue_roofline(reb_s, seg_s, pairs, clocks):
         out["stale"] = "kernel sources differ from the profiled ones: no instruction count for this code"
         return out
     out["profiled_sources_sha256"] = prof["sources_sha256"]
-    for name, t in (("k_rebuild", reb_s), ("k_segments", seg_s)):
+    for name, t in (("k_rebuild_team", reb_s), ("k_segments", seg_s)):
         inst = float(prof[name]["warp_inst_per_pair"]) * pairs
         out[name] = {"bound": "issue", "achieved": inst / t, "frac": inst / t / peak, "warp_inst_per_launch": inst}
     return out
@@ -552,7 +552,7 @@ def _sweep_line(args, world, value, T, totals, launches, clk, wall, e2e_value, h
     achieved = abytes / seg_s / 1e9
     prof = profiled_current()
     traffic = prof["k_segments"]["dram_bytes_per_pair"] * args.pairs if prof else None
-    reb_traffic = prof["k_rebuild"]["dram_bytes_per_pair"] * args.pairs if prof else None
+    reb_traffic = prof["k_rebuild_team"]["dram_bytes_per_pair"] * args.pairs if prof else None
     cfg = dict(base_cfg)
     cfg.update({"l2": "flushed (256 MB write) before every timed step", "inputs": "device-resident for value",
                 "contacts_per_step": int(totals[0]), "segments_per_step": int(totals[1]),
@@ -564,7 +564,7 @@ def _sweep_line(args, world, value, T, totals, launches, clk, wall, e2e_value, h
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": reb_bytes / reb_s / 1e9, "peak": peak, "unit": "GB/s",
-                         "frac": reb_bytes / reb_s / 1e9 / peak, "traffic": reb_traffic, "kernel": "k_rebuild",
+                         "frac": reb_bytes / reb_s / 1e9 / peak, "traffic": reb_traffic, "kernel": "k_rebuild_team",
                          "peak_kind": f"{peak_kind} hbm_gbs", "algorithmic_bytes_per_launch": reb_bytes,
                          "kernel_ms": 1e3 * reb_s,
                          "note": "latency bound (serial per-pair topology in the reference's order); see profiles/"},

@@ -8,8 +8,8 @@
 //   * box tests of all segment pairs (32 x 32 tiles, outward-rounded floats) list the few that overlap;
 //     lanes over that list take the cell ranks, the endpoint distances and the segment distances;
 //   * components by a lock-free union-find over the accepted pairs.  The search order inside a component
-//     (src/main.cpp:874-897) is then one thread's depth-first walk over sorted neighbour lists, all
-//     components at once;
+//     (src/main.cpp:874-897) is then a depth-first walk over sorted neighbour lists, a warp a
+//     component, its lanes over the list of the segment popped;
 //   * the snap is a union-find over the endpoints of listed pairs (two endpoints within h lie in adjacent
 //     cells, so their segments are listed); links point at the smaller endpoint, so a class's root is its
 //     first appearance and vertex ids are a scan;

@@ -2,15 +2,16 @@
 
 The knobs change how the batched pair call is launched, never what it computes:
 
-* ``tri_ctas_per_sm``  triangle-stage CTAs resident per SM (each holds one pair's survivors);
+* ``tri_ctas_per_sm``  triangle-stage CTAs resident per SM (each holds one pair's survivors): one, or as
+                       many as fit (2);
 * ``flat_max``         survivor pairs nA' x nB' up to which the triangle stage tests every box pair
                        directly, above which it uses the Morton-ordered group boxes;
-* ``rebuild_warps``    warps per rebuild block (one warp per pair);
+* ``rebuild_warps``    warps per rebuild block, where a warp takes a pair;
 * ``split_tests``      in a batch with fewer pairs than triangle-stage CTAs, the triangle tests per work
                        item into which large pairs are split (0: no split);
-* ``rebuild_arena``    the rebuild's form: one warp per pair over global-memory slots (0), the large
-                       pairs in arenas alongside form 0 on the small ones (1), or arenas for every
-                       pair (2);
+* ``rebuild_arena``    the rebuild's form: packs of pairs in shared memory, and one warp per pair over
+                       global-memory slots for the pairs no block holds (0), the large pairs in arenas
+                       alongside the warps on the small ones (1), or arenas for every pair (2);
 * ``arena_warps``      warps per SM given arenas;
 * ``arena_min_seg``    the segment count from which form 1 gives a pair an arena.
 
